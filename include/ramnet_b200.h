@@ -23,6 +23,8 @@ extern "C" {
 #endif
 
 enum { RN_F32 = 0, RN_F16 = 1, RN_BF16 = 2 };
+/* Token positions: int32, int64 (the low 32 bits count), or the index of the token in the call (no tensor). */
+enum { RN_POS_I32 = 0, RN_POS_I64 = 1, RN_POS_INDEX = 2 };
 
 /* Width of the index type used for slot indices (the reference exports the same number as
  * ramnet_ops._C.INT_BITS, packages/ramnet-ops/csrc/ram_attn_bind.cpp:120-129).  State element
@@ -87,6 +89,13 @@ int rn_addr_fwd(const void *w_addr, const void *r_addr, int dtype, const int64_t
                 int64_t B, int64_t H, int64_t U, int64_t P, int64_t T, int64_t E,
                 int64_t Kw, int64_t Kr, double w_re_norm, double r_re_norm,
                 int w_neg, int r_neg, int encode_batch, int device, void *stream);
+/* The same with positions in any of the RN_POS_* forms (pos and pos_strides may be NULL for RN_POS_INDEX). */
+int rn_addr_fwd_pos(const void *w_addr, const void *r_addr, int dtype, const int64_t *addr_strides,
+                    const void *pos, int pos_kind, const int64_t *pos_strides,
+                    int32_t *idx, float *val, const int64_t *out_strides,
+                    int64_t B, int64_t H, int64_t U, int64_t P, int64_t T, int64_t E,
+                    int64_t Kw, int64_t Kr, double w_re_norm, double r_re_norm,
+                    int w_neg, int r_neg, int encode_batch, int device, void *stream);
 
 /*
  * Gradient of the decoded weights w.r.t. the logits.
@@ -109,6 +118,14 @@ int rn_addr_bwd(const int32_t *idx, const float *val, const int64_t *out_strides
                 int64_t B, int64_t H, int64_t U, int64_t P, int64_t T, int64_t E,
                 int64_t Kw, int64_t Kr, double w_re_norm, double r_re_norm,
                 int w_neg, int r_neg, int device, void *stream);
+int rn_addr_bwd_pos(const int32_t *idx, const float *val, const int64_t *out_strides,
+                    const float *d_val, const int64_t *dval_strides,
+                    const void *w_addr, const void *r_addr, int dtype, const int64_t *addr_strides,
+                    const void *pos, int pos_kind, const int64_t *pos_strides,
+                    void *d_w, void *d_r, const int64_t *dgrad_strides,
+                    int64_t B, int64_t H, int64_t U, int64_t P, int64_t T, int64_t E,
+                    int64_t Kw, int64_t Kr, double w_re_norm, double r_re_norm,
+                    int w_neg, int r_neg, int device, void *stream);
 
 /*
  * One fused autoregressive decode step: address decode for the write and read logits, gated
@@ -153,6 +170,14 @@ int rn_decode_step_scaled(const void *w_addr, const void *r_addr, const void *x,
                           int64_t B, int64_t H, int64_t U, int64_t P, int64_t C, int64_t E,
                           int64_t Kw, int64_t Kr, double w_re_norm, double r_re_norm,
                           int mass_aware, double eps, int device, void *stream);
+/* The same with positions in any of the RN_POS_* forms, pos_stride elements between batch rows. */
+int rn_decode_step_pos(const void *w_addr, const void *r_addr, const void *x, const void *gamma, int dtype,
+                       float *slot, float *mass, const uint8_t *mask, const void *pos, int pos_kind, int64_t pos_stride,
+                       void *y, const float *norm_weight, const void *gate_logits, double norm_eps,
+                       const void *w_scale, const void *r_scale, const int64_t *batch_strides,
+                       int64_t B, int64_t H, int64_t U, int64_t P, int64_t C, int64_t E,
+                       int64_t Kw, int64_t Kr, double w_re_norm, double r_re_norm,
+                       int mass_aware, double eps, int device, void *stream);
 
 /*
  * Prefill (T > 1) gated sparse update + read over decoded addresses.
@@ -206,6 +231,14 @@ int rn_gsu_fwd(const int32_t *idx, const float *val, const int64_t *idx_strides,
                float *slot_out, float *mass_out, void *y, const int64_t *y_strides, void *workspace,
                int64_t workspace_bytes, int64_t B, int64_t H, int64_t T, int64_t A, int64_t C, int64_t Kw,
                int64_t Kr, int mass_aware, double eps, int device, void *stream);
+/* The same for a state that does not exist yet: slot_in == NULL stands for rows of zeros, mass_in == NULL for
+ * mass_init in every slot, so that nobody fills and reads back a fresh state. */
+int rn_gsu_fwd_init(const int32_t *idx, const float *val, const int64_t *idx_strides, const void *x,
+                    const int64_t *x_strides, const void *gamma, const int64_t *gamma_strides, int dtype,
+                    const uint8_t *mask, const int64_t *mask_strides, const float *slot_in, const float *mass_in,
+                    double mass_init, float *slot_out, float *mass_out, void *y, const int64_t *y_strides,
+                    void *workspace, int64_t workspace_bytes, int64_t B, int64_t H, int64_t T, int64_t A, int64_t C,
+                    int64_t Kw, int64_t Kr, int mass_aware, double eps, int device, void *stream);
 
 /*
  * Backward of the prefill update / read (plain and mass-aware reads).

@@ -10,8 +10,7 @@
 struct RnAddrFwdParams {
     const void *addr[2];
     int64_t sb, sh, su, sp, st;
-    const int32_t *pos;
-    int64_t pb, pt;
+    RnPos pos;
     int32_t *idx;
     float *val;
     int64_t ob, oh, ok, ot;
@@ -53,7 +52,7 @@ __global__ void __launch_bounds__(RN_ADDR_WARPS * 32) rn_addr_fwd_kernel(const R
         const int K = p.K[which];
         const RnDecoded<KPL> d = rn_warp_decode<KPL, PPL>(load, p.U, p.P, K, p.re_norm[which], ws, &tabs[which], lane);
 
-        const int shift = (h < p.E) ? rn_pos_mod(p.pos[b * p.pb + t * p.pt], p.A) : 0;
+        const int shift = (h < p.E) ? rn_pos_mod(rn_pos_at(p.pos, b, t), p.A) : 0;
         const int offs = (p.encode_batch ? (b * p.H + h) : h) * p.A;
         const int koff = which ? p.K[0] : 0;
         const int64_t obase = b * p.ob + h * p.oh + t * p.ot;
@@ -80,8 +79,7 @@ struct RnAddrBwdParams {
     int64_t gb, gh, gk, gt;
     const void *addr[2];
     int64_t sb, sh, su, sp, st;
-    const int32_t *pos;
-    int64_t pb, pt;
+    RnPos pos;
     void *d_addr[2];
     int64_t db, dh, du, dp, dt;
     int B, H, U, P, T, E, A;
@@ -115,7 +113,7 @@ __global__ void __launch_bounds__(RN_ADDR_WARPS * 32) rn_addr_bwd_kernel(const R
         const int K = p.K[which];
         const int koff = which ? p.K[0] : 0;
         const float rho = p.re_norm[which];
-        const int shift = (h < p.E) ? rn_pos_mod(p.pos[b * p.pb + t * p.pt], p.A) : 0;
+        const int shift = (h < p.E) ? rn_pos_mod(rn_pos_at(p.pos, b, t), p.A) : 0;
 
         float dsum = 0.f, wsum = 0.f;
         for (int k = lane; k < K; k += 32) {
@@ -248,22 +246,41 @@ static int rn_launch_addr_fwd(const RnAddrFwdParams &p, int kpl, int ppl, int gr
     return 1;
 }
 
+// the positions of a call; null strides (or RN_POS_INDEX) need no tensor
+static RnPos rn_make_pos(const void *pos, int kind, const int64_t *strides) {
+    RnPos q{pos, 0, 0, kind};
+    if (strides != nullptr) { q.sb = strides[0]; q.st = strides[1]; }
+    return q;
+}
+
 extern "C" int rn_addr_fwd(const void *w_addr, const void *r_addr, int dtype, const int64_t *addr_strides,
                            const int32_t *pos, const int64_t *pos_strides, int32_t *idx, float *val,
                            const int64_t *out_strides, int64_t B, int64_t H, int64_t U, int64_t P, int64_t T, int64_t E,
                            int64_t Kw, int64_t Kr, double w_re_norm, double r_re_norm, int w_neg, int r_neg,
                            int encode_batch, int device, void *stream) {
+    return rn_addr_fwd_pos(w_addr, r_addr, dtype, addr_strides, pos, RN_POS_I32, pos_strides, idx, val, out_strides, B, H, U, P,
+                           T, E, Kw, Kr, w_re_norm, r_re_norm, w_neg, r_neg, encode_batch, device, stream);
+}
+
+extern "C" int rn_addr_fwd_pos(const void *w_addr, const void *r_addr, int dtype, const int64_t *addr_strides,
+                               const void *pos_, int pos_kind, const int64_t *pos_strides, int32_t *idx, float *val,
+                               const int64_t *out_strides, int64_t B, int64_t H, int64_t U, int64_t P, int64_t T,
+                               int64_t E, int64_t Kw, int64_t Kr, double w_re_norm, double r_re_norm, int w_neg,
+                               int r_neg, int encode_batch, int device, void *stream) {
     rn_clear_error();
     int64_t A = 0;
     if (int rc = rn_check_addr_dims(B, H, U, P, T, E, Kw, Kr, w_re_norm, r_re_norm, dtype, &A)) return rc;
-    RN_REQUIRE(w_addr && pos && idx && val && addr_strides && pos_strides && out_strides, "null pointer argument");
+    RN_REQUIRE(pos_kind >= RN_POS_I32 && pos_kind <= RN_POS_INDEX, "unknown kind of positions: %d", pos_kind);
+    RN_REQUIRE(w_addr && (pos_kind == RN_POS_INDEX || (pos_ && pos_strides)) && idx && val && addr_strides && out_strides,
+               "null pointer argument");
+    const RnPos pos = rn_make_pos(pos_, pos_kind, pos_strides);
     RN_REQUIRE((r_addr != nullptr) == (Kr > 0), "r_addr must be given exactly when r_top_k > 0");
     RnDeviceGuard guard(device);
     RN_REQUIRE(guard.ok, "cannot make device %d current", device);
 
     rn_prof_reset();
     rn_prof_mark(cudaStream_t(stream));
-    if (rn_addr_fwd_fast(w_addr, r_addr, dtype, addr_strides, pos, pos_strides, idx, val, out_strides, B, H, U, P, T, E, A,
+    if (rn_addr_fwd_fast(w_addr, r_addr, dtype, addr_strides, pos, idx, val, out_strides, B, H, U, P, T, E, A,
                          Kw, Kr, w_re_norm, r_re_norm, w_neg, r_neg, encode_batch, cudaStream_t(stream)) == 0) {
         RN_CUDA(cudaGetLastError());
         rn_prof_mark(cudaStream_t(stream));
@@ -274,7 +291,7 @@ extern "C" int rn_addr_fwd(const void *w_addr, const void *r_addr, int dtype, co
     p.addr[0] = w_addr;
     p.addr[1] = r_addr;
     p.sb = addr_strides[0]; p.sh = addr_strides[1]; p.su = addr_strides[2]; p.sp = addr_strides[3]; p.st = addr_strides[4];
-    p.pos = pos; p.pb = pos_strides[0]; p.pt = pos_strides[1];
+    p.pos = pos;
     p.idx = idx; p.val = val;
     p.ob = out_strides[0]; p.oh = out_strides[1]; p.ok = out_strides[2]; p.ot = out_strides[3];
     p.B = int(B); p.H = int(H); p.U = int(U); p.P = int(P); p.T = int(T); p.E = int(E); p.A = int(A);
@@ -315,12 +332,25 @@ extern "C" int rn_addr_bwd(const int32_t *idx, const float *val, const int64_t *
                            void *d_r, const int64_t *dgrad_strides, int64_t B, int64_t H, int64_t U, int64_t P,
                            int64_t T, int64_t E, int64_t Kw, int64_t Kr, double w_re_norm, double r_re_norm, int w_neg,
                            int r_neg, int device, void *stream) {
+    return rn_addr_bwd_pos(idx, val, out_strides, d_val, dval_strides, w_addr, r_addr, dtype, addr_strides, pos, RN_POS_I32,
+                           pos_strides, d_w, d_r, dgrad_strides, B, H, U, P, T, E, Kw, Kr, w_re_norm, r_re_norm, w_neg, r_neg,
+                           device, stream);
+}
+
+extern "C" int rn_addr_bwd_pos(const int32_t *idx, const float *val, const int64_t *out_strides, const float *d_val,
+                           const int64_t *dval_strides, const void *w_addr, const void *r_addr, int dtype,
+                           const int64_t *addr_strides, const void *pos_, int pos_kind, const int64_t *pos_strides, void *d_w,
+                           void *d_r, const int64_t *dgrad_strides, int64_t B, int64_t H, int64_t U, int64_t P,
+                           int64_t T, int64_t E, int64_t Kw, int64_t Kr, double w_re_norm, double r_re_norm, int w_neg,
+                           int r_neg, int device, void *stream) {
     rn_clear_error();
     int64_t A = 0;
     if (int rc = rn_check_addr_dims(B, H, U, P, T, E, Kw, Kr, w_re_norm, r_re_norm, dtype, &A)) return rc;
-    RN_REQUIRE(idx && val && d_val && w_addr && pos && d_w && out_strides && dval_strides && addr_strides &&
-                   pos_strides && dgrad_strides,
+    RN_REQUIRE(pos_kind >= RN_POS_I32 && pos_kind <= RN_POS_INDEX, "unknown kind of positions: %d", pos_kind);
+    RN_REQUIRE(idx && val && d_val && w_addr && (pos_kind == RN_POS_INDEX || (pos_ && pos_strides)) && d_w && out_strides &&
+                   dval_strides && addr_strides && dgrad_strides,
                "null pointer argument");
+    const RnPos pos = rn_make_pos(pos_, pos_kind, pos_strides);
     RN_REQUIRE((r_addr != nullptr) == (Kr > 0) && (d_r != nullptr) == (Kr > 0),
                "r_addr and d_r must be given exactly when r_top_k > 0");
     RnDeviceGuard guard(device);
@@ -328,7 +358,7 @@ extern "C" int rn_addr_bwd(const int32_t *idx, const float *val, const int64_t *
 
     rn_prof_reset();
     rn_prof_mark(cudaStream_t(stream));
-    if (rn_addr_bwd_fast(idx, val, out_strides, d_val, dval_strides, w_addr, r_addr, dtype, addr_strides, pos, pos_strides,
+    if (rn_addr_bwd_fast(idx, val, out_strides, d_val, dval_strides, w_addr, r_addr, dtype, addr_strides, pos,
                          d_w, d_r, dgrad_strides, B, H, U, P, T, E, A, Kw, Kr, w_re_norm, r_re_norm, w_neg, r_neg,
                          cudaStream_t(stream)) == 0) {
         RN_CUDA(cudaGetLastError());
@@ -343,7 +373,7 @@ extern "C" int rn_addr_bwd(const int32_t *idx, const float *val, const int64_t *
     p.gb = dval_strides[0]; p.gh = dval_strides[1]; p.gk = dval_strides[2]; p.gt = dval_strides[3];
     p.addr[0] = w_addr; p.addr[1] = r_addr;
     p.sb = addr_strides[0]; p.sh = addr_strides[1]; p.su = addr_strides[2]; p.sp = addr_strides[3]; p.st = addr_strides[4];
-    p.pos = pos; p.pb = pos_strides[0]; p.pt = pos_strides[1];
+    p.pos = pos;
     p.d_addr[0] = d_w; p.d_addr[1] = d_r;
     p.db = dgrad_strides[0]; p.dh = dgrad_strides[1]; p.du = dgrad_strides[2]; p.dp = dgrad_strides[3]; p.dt = dgrad_strides[4];
     p.B = int(B); p.H = int(H); p.U = int(U); p.P = int(P); p.T = int(T); p.E = int(E); p.A = int(A);

@@ -9,8 +9,7 @@ using namespace rn_fast;
 struct FastParams {
     const void *addr[2];
     int64_t sb, sh, st;      // element strides of batch / head / token; the U*P block is contiguous
-    const int32_t *pos;
-    int64_t pb, pt;
+    RnPos pos;
     int32_t *idx;
     float *val;
     int64_t ob, oh, ot;      // output strides; the K entries of a row are contiguous
@@ -39,7 +38,7 @@ __global__ void __launch_bounds__(FAST_THREADS) rn_addr_fast_kernel(const FastPa
     int content[K];
     float weight[K];
     thread_decode<T, U, P, K>(src, p.re_norm[which], content, weight);
-    const int shift = (h < p.E) ? rn_pos_mod(p.pos[b * p.pb + t * p.pt], p.A) : 0;
+    const int shift = (h < p.E) ? rn_pos_mod(rn_pos_at(p.pos, b, t), p.A) : 0;
     const int offs = (p.encode_batch ? (b * p.H + h) : h) * p.A;
     const int64_t o = b * p.ob + h * p.oh + t * p.ot + (which ? K : 0);
     int out_i[K];
@@ -93,8 +92,7 @@ struct FastBwdParams {
     int64_t sb, sh, st;
     void *d_addr[2];
     int64_t db, dh, dt;
-    const int32_t *pos;
-    int64_t pb, pt;
+    RnPos pos;
     int B, H, T, E, A;
     float re_norm[2];
     float sign[2];
@@ -167,7 +165,7 @@ __global__ void __launch_bounds__(FAST_THREADS) rn_addr_bwd_fast_kernel(const Fa
     const int t = int((row / p.H) % p.T);
     const int b = int(row / (int64_t(p.H) * p.T));
     const float rho = p.re_norm[which];
-    const int shift = (h < p.E) ? rn_pos_mod(p.pos[b * p.pb + t * p.pt], p.A) : 0;
+    const int shift = (h < p.E) ? rn_pos_mod(rn_pos_at(p.pos, b, t), p.A) : 0;
     // the lanes of a row are LPR consecutive lanes of one warp
     const unsigned gmask = (LPR >= 32 ? 0xffffffffu : ((1u << LPR) - 1u)) << ((tid & 31) & ~(LPR - 1));
 
@@ -282,8 +280,8 @@ int dispatch_bwd_fast(const FastBwdParams &p, int U, int P, int K, cudaStream_t 
 }  // namespace
 
 // Returns 0 when a specialised kernel was launched, -1 when the shape / layout has none.
-int rn_addr_fwd_fast(const void *w_addr, const void *r_addr, int dtype, const int64_t *addr_strides, const int32_t *pos,
-                     const int64_t *pos_strides, int32_t *idx, float *val, const int64_t *out_strides, int64_t B,
+int rn_addr_fwd_fast(const void *w_addr, const void *r_addr, int dtype, const int64_t *addr_strides, const RnPos &pos,
+                     int32_t *idx, float *val, const int64_t *out_strides, int64_t B,
                      int64_t H, int64_t U, int64_t P, int64_t T, int64_t E, int64_t A, int64_t Kw, int64_t Kr,
                      double w_re_norm, double r_re_norm, int w_neg, int r_neg, int encode_batch, cudaStream_t stream) {
     if (r_addr != nullptr && Kw != Kr) return -1;
@@ -302,7 +300,7 @@ int rn_addr_fwd_fast(const void *w_addr, const void *r_addr, int dtype, const in
     FastParams p{};
     p.addr[0] = w_addr; p.addr[1] = r_addr;
     p.sb = addr_strides[0]; p.sh = addr_strides[1]; p.st = addr_strides[4];
-    p.pos = pos; p.pb = pos_strides[0]; p.pt = pos_strides[1];
+    p.pos = pos;
     p.idx = idx; p.val = val;
     p.ob = out_strides[0]; p.oh = out_strides[1]; p.ot = out_strides[3];
     p.B = int(B); p.H = int(H); p.T = int(T); p.E = int(E); p.A = int(A);
@@ -319,7 +317,7 @@ int rn_addr_fwd_fast(const void *w_addr, const void *r_addr, int dtype, const in
 // Backward of the address decode for the same shapes and layouts; 0 = launched, -1 = use the general kernel.
 int rn_addr_bwd_fast(const int32_t *idx, const float *val, const int64_t *out_strides, const float *d_val,
                      const int64_t *dval_strides, const void *w_addr, const void *r_addr, int dtype,
-                     const int64_t *addr_strides, const int32_t *pos, const int64_t *pos_strides, void *d_w, void *d_r,
+                     const int64_t *addr_strides, const RnPos &pos, void *d_w, void *d_r,
                      const int64_t *dgrad_strides, int64_t B, int64_t H, int64_t U, int64_t P, int64_t T, int64_t E,
                      int64_t A, int64_t Kw, int64_t Kr, double w_re_norm, double r_re_norm, int w_neg, int r_neg,
                      cudaStream_t stream) {
@@ -351,7 +349,7 @@ int rn_addr_bwd_fast(const int32_t *idx, const float *val, const int64_t *out_st
     p.sb = addr_strides[0]; p.sh = addr_strides[1]; p.st = addr_strides[4];
     p.d_addr[0] = d_w; p.d_addr[1] = d_r;
     p.db = dgrad_strides[0]; p.dh = dgrad_strides[1]; p.dt = dgrad_strides[4];
-    p.pos = pos; p.pb = pos_strides[0]; p.pt = pos_strides[1];
+    p.pos = pos;
     p.B = int(B); p.H = int(H); p.T = int(T); p.E = int(E); p.A = int(A);
     p.re_norm[0] = float(w_re_norm); p.re_norm[1] = float(r_re_norm);
     p.sign[0] = w_neg ? -1.f : 1.f; p.sign[1] = r_neg ? -1.f : 1.f;

@@ -63,6 +63,20 @@ void rn_prof_mark(cudaStream_t stream);
 // ------------------------------------------------------------------------------------------
 constexpr unsigned RN_FULL = 0xffffffffu;
 
+// Token positions as the caller keeps them (RN_POS_*): 32-bit, 64-bit (the low 32 bits count, as after a conversion to
+// int32), or the token index itself.  Read in place: a conversion kernel in front of a decode step costs as much as a
+// tenth of the step.
+struct RnPos {
+    const void *p;
+    int64_t sb, st;  // element strides over (batch, token)
+    int kind;
+};
+__device__ __forceinline__ int rn_pos_at(const RnPos &q, int b, int t) {
+    if (q.kind == RN_POS_INDEX) return t;
+    const int64_t o = b * q.sb + t * q.st;
+    return q.kind == RN_POS_I64 ? int(static_cast<const long long *>(q.p)[o]) : static_cast<const int32_t *>(q.p)[o];
+}
+
 template <typename T> __device__ __forceinline__ float rn_to_float(T v);
 template <> __device__ __forceinline__ float rn_to_float<float>(float v) { return v; }
 template <> __device__ __forceinline__ float rn_to_float<__half>(__half v) { return __half2float(v); }

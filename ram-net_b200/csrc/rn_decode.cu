@@ -27,7 +27,7 @@ struct RnDecodeParams {
     const void *w_addr, *r_addr, *x, *gamma;
     float *slot, *mass;
     const uint8_t *mask;
-    const int32_t *pos;
+    RnPos pos;
     void *y;
     const float *norm_weight;
     const void *gate;
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(RN_DEC_WARPS * 32) rn_decode_kernel(const RnDe
         const int K = p.K[warp];
         const RnDecoded<KPL> d =
             rn_warp_decode<KPL, PPL>(load, p.U, p.P, K, p.re_norm[warp], &scratch[warp], warp == 0 ? &tabs[0] : tab_r, lane);
-        const int shift = (h < p.E) ? rn_pos_mod(p.pos[b], p.A) : 0;
+        const int shift = (h < p.E) ? rn_pos_mod(rn_pos_at(p.pos, b, 0), p.A) : 0;
 #pragma unroll
         for (int r = 0; r < KPL; ++r) {
             const int e = lane * KPL + r;
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(RN_DECF_THREADS, 2) rn_decode_fast_kernel(cons
         float weight[K];
         rn_fast::quad_decode<T, U, P, K>(src, p.re_norm[which], gl, content, weight);
         if (gl == 0 && bh0 + pair < BH) {
-            const int shift = (h < p.E) ? rn_pos_mod(p.pos[b], p.A) : 0;
+            const int shift = (h < p.E) ? rn_pos_mod(rn_pos_at(p.pos, b, 0), p.A) : 0;
 #pragma unroll
             for (int e = 0; e < K; ++e) {
                 sel_slot[pair][which][e] = rn_cape(content[e], shift, p.A);
@@ -520,7 +520,7 @@ __device__ __forceinline__ uint32_t rn_decode_pair_task(const RnDecodeParams &p,
 
         // inputs that do not depend on the addresses are requested first
         const float gamma = rn_to_float<T>(static_cast<const T *>(p.gamma)[(EXTRA ? rn_in_row(p, bh, p.ld_gamma, 1) : int64_t(bh) * (1))]);
-        const int shift = (h < p.E) ? rn_pos_mod(p.pos[b], p.A) : 0;
+        const int shift = (h < p.E) ? rn_pos_mod(rn_pos_at(p.pos, b, 0), p.A) : 0;
         RnRaw4<T> xraw[NV];
 #pragma unroll
         for (int v = 0; v < NV; ++v) xraw[v] = rn_load_raw4<T>(static_cast<const T *>(p.x) + (EXTRA ? rn_in_row(p, bh, p.ld_x, C) : int64_t(bh) * (C)) + v * 128 + lane * 4);
@@ -811,13 +811,6 @@ static int rn_launch_decode(const RnDecodeParams &p, int kpl, int ppl, int grid,
     return 1;
 }
 
-extern "C" int rn_decode_step_scaled(const void *w_addr, const void *r_addr, const void *x, const void *gamma, int dtype,
-                                     float *slot, float *mass, const uint8_t *mask, const int32_t *pos, void *y,
-                                     const float *norm_weight, const void *gate_logits, double norm_eps,
-                                     const void *w_scale, const void *r_scale, const int64_t *batch_strides, int64_t B,
-                                     int64_t H, int64_t U, int64_t P, int64_t C, int64_t E, int64_t Kw, int64_t Kr,
-                                     double w_re_norm, double r_re_norm, int mass_aware, double eps, int device, void *stream);
-
 // 1 when rn_decode_step_scaled() takes logit scales for this shape (the one-warp-per-pair kernel does), else 0
 extern "C" int rn_decode_scales_supported(int dtype, int64_t U, int64_t P, int64_t C, int64_t Kw, int64_t Kr) {
     return (dtype == RN_F16 || dtype == RN_BF16) && U == 2 && P == 64 && Kw == 16 && Kr == 16 && (C == 128 || C == 256);
@@ -839,11 +832,23 @@ extern "C" int rn_decode_step_scaled(const void *w_addr, const void *r_addr, con
                                      const void *w_scale, const void *r_scale, const int64_t *batch_strides, int64_t B,
                                      int64_t H, int64_t U, int64_t P, int64_t C, int64_t E, int64_t Kw, int64_t Kr,
                                      double w_re_norm, double r_re_norm, int mass_aware, double eps, int device, void *stream) {
+    return rn_decode_step_pos(w_addr, r_addr, x, gamma, dtype, slot, mass, mask, pos, RN_POS_I32, 1, y, norm_weight, gate_logits,
+                              norm_eps, w_scale, r_scale, batch_strides, B, H, U, P, C, E, Kw, Kr, w_re_norm, r_re_norm,
+                              mass_aware, eps, device, stream);
+}
+
+extern "C" int rn_decode_step_pos(const void *w_addr, const void *r_addr, const void *x, const void *gamma, int dtype,
+                                  float *slot, float *mass, const uint8_t *mask, const void *pos, int pos_kind,
+                                  int64_t pos_stride, void *y, const float *norm_weight, const void *gate_logits,
+                                  double norm_eps, const void *w_scale, const void *r_scale, const int64_t *batch_strides,
+                                  int64_t B, int64_t H, int64_t U, int64_t P, int64_t C, int64_t E, int64_t Kw, int64_t Kr,
+                                  double w_re_norm, double r_re_norm, int mass_aware, double eps, int device, void *stream) {
     rn_clear_error();
+    RN_REQUIRE(pos_kind >= RN_POS_I32 && pos_kind <= RN_POS_INDEX, "unknown kind of positions: %d", pos_kind);
     RN_REQUIRE((w_scale == nullptr) == (r_scale == nullptr), "give both logit scales or none");
     RN_REQUIRE(w_scale == nullptr || rn_decode_scales_supported(dtype, U, P, C, Kw, Kr),
                "logit scales are taken for 16-bit logits with U=2, P=64, K=16, C in {128, 256} only");
-    RN_REQUIRE(w_addr && r_addr && x && gamma && slot && mass && pos && y, "null pointer argument");
+    RN_REQUIRE(w_addr && r_addr && x && gamma && slot && mass && (pos || pos_kind == RN_POS_INDEX) && y, "null pointer argument");
     RN_REQUIRE(B > 0 && H > 0 && U > 0 && P > 0 && C > 0, "decode dims must be positive");
     RN_REQUIRE(U <= RN_UMAX, "Expect U <= %d but got %lld", RN_UMAX, (long long)U);
     RN_REQUIRE(P <= RN_PMAX, "Expect P <= %d but got %lld", RN_PMAX, (long long)P);
@@ -866,7 +871,8 @@ extern "C" int rn_decode_step_scaled(const void *w_addr, const void *r_addr, con
 
     RnDecodeParams p{};
     p.w_addr = w_addr; p.r_addr = r_addr; p.x = x; p.gamma = gamma;
-    p.slot = slot; p.mass = mass; p.mask = mask; p.pos = pos; p.y = y;
+    p.slot = slot; p.mass = mass; p.mask = mask; p.y = y;
+    p.pos = RnPos{pos, pos_stride, 0, pos_kind};
     p.norm_weight = norm_weight; p.gate = gate_logits; p.norm_eps = float(norm_eps);
     p.scale[0] = w_scale; p.scale[1] = r_scale;
     p.ld_addr[0] = batch_strides ? batch_strides[0] : H * U * P;

@@ -47,9 +47,9 @@ __global__ void __launch_bounds__(RN_SCHED_THREADS_MAX) rn_gsu_schedule_kernel(c
     float *ev_v = reinterpret_cast<float *>(cur);
     float *ev_c = ev_v + p.NE;
 
-    const float *mass_in = p.mass_in + int64_t(bh) * A;
+    const float *mass_in = p.mass_in ? p.mass_in + int64_t(bh) * A : nullptr;
     for (int a = tid; a < A; a += NT) {
-        if (SMEM_TABLES || mass_in != mass) mass[a] = mass_in[a];
+        if (SMEM_TABLES || mass_in != mass) mass[a] = mass_in ? mass_in[a] : p.mass_init;
         claim[a] = 0xffffffffu;
     }
 
@@ -318,10 +318,10 @@ __global__ void __launch_bounds__(RN_GSU_THREADS) rn_gsu_apply_kernel(const RnGs
         S = cur;
         cur += size_t(A) * cs;
         srow = cs;
-        const float *src = p.slot_in + int64_t(bh) * A * C + c0;
+        const float *src = p.slot_in ? p.slot_in + int64_t(bh) * A * C + c0 : nullptr;
         for (int i = tid; i < A * cs; i += RN_GSU_THREADS) {
             const int a = i / cs, c = i - a * cs;
-            S[i] = c < cvalid ? src[int64_t(a) * C + c] : 0.f;
+            S[i] = src != nullptr && c < cvalid ? src[int64_t(a) * C + c] : 0.f;
         }
     } else {
         S = p.slot_out + int64_t(bh) * A * C + c0;  // holds the initial state already
@@ -492,11 +492,11 @@ __global__ void __launch_bounds__(RN_APPLY_THREADS, 1) rn_gsu_apply_fast_kernel(
 
     // state slice -> shared memory
     {
-        const float *src = p.slot_in + int64_t(bh) * A * C + c0;
+        const float *src = p.slot_in ? p.slot_in + int64_t(bh) * A * C + c0 : nullptr;
         for (int i = tid; i < A * G; i += RN_APPLY_THREADS) {
             const int a = i / G, sg = i - a * G;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (sg * 4 < cvalid) v = *reinterpret_cast<const float4 *>(src + int64_t(a) * C + sg * 4);
+            if (src != nullptr && sg * 4 < cvalid) v = *reinterpret_cast<const float4 *>(src + int64_t(a) * C + sg * 4);
             *reinterpret_cast<float4 *>(S + rn_row_of_slot(uint32_t(a), A, p.row_shift) * CS + sg * 4) = v;
         }
     }
@@ -883,8 +883,21 @@ extern "C" int rn_gsu_fwd(const int32_t *idx, const float *val, const int64_t *i
                           int64_t workspace_bytes, int64_t B, int64_t H, int64_t T, int64_t A, int64_t C, int64_t Kw,
                           int64_t Kr, int mass_aware, double eps, int device, void *stream_) {
     rn_clear_error();
-    RN_REQUIRE(idx && val && idx_strides && x && x_strides && gamma && gamma_strides && slot_in && mass_in && slot_out &&
-                   mass_out && y && y_strides,
+    RN_REQUIRE(slot_in && mass_in, "null pointer argument");
+    return rn_gsu_fwd_init(idx, val, idx_strides, x, x_strides, gamma, gamma_strides, dtype, mask, mask_strides, slot_in, mass_in,
+                           0.0, slot_out, mass_out, y, y_strides, workspace, workspace_bytes, B, H, T, A, C, Kw, Kr, mass_aware,
+                           eps, device, stream_);
+}
+
+extern "C" int rn_gsu_fwd_init(const int32_t *idx, const float *val, const int64_t *idx_strides, const void *x,
+                               const int64_t *x_strides, const void *gamma, const int64_t *gamma_strides, int dtype,
+                               const uint8_t *mask, const int64_t *mask_strides, const float *slot_in,
+                               const float *mass_in, double mass_init, float *slot_out, float *mass_out, void *y,
+                               const int64_t *y_strides, void *workspace, int64_t workspace_bytes, int64_t B, int64_t H,
+                               int64_t T, int64_t A, int64_t C, int64_t Kw, int64_t Kr, int mass_aware, double eps,
+                               int device, void *stream_) {
+    rn_clear_error();
+    RN_REQUIRE(idx && val && idx_strides && x && x_strides && gamma && gamma_strides && slot_out && mass_out && y && y_strides,
                "null pointer argument");
     RN_REQUIRE(dtype == RN_F32 || dtype == RN_F16 || dtype == RN_BF16, "unsupported dtype code %d", dtype);
     RN_REQUIRE(x_strides[3] == 1 && y_strides[3] == 1, "Tensor x / y last dim must be contiguous");
@@ -898,7 +911,7 @@ extern "C" int rn_gsu_fwd(const int32_t *idx, const float *val, const int64_t *i
     cudaStream_t stream = cudaStream_t(stream_);
 
     // model shapes: the slot-owner kernel (one cluster per (b,h)), which needs no schedule and no workspace
-    if (rn_gsu_owner_eligible(dtype, A, C, Kw, Kr, x, x_strides, y, y_strides)) {
+    if (slot_in && mass_in && rn_gsu_owner_eligible(dtype, A, C, Kw, Kr, x, x_strides, y, y_strides)) {
         RnGsuParams q{};
         q.idx = idx; q.val = val;
         q.ib = idx_strides[0]; q.ih = idx_strides[1]; q.ik = idx_strides[2]; q.it = idx_strides[3];
@@ -935,7 +948,7 @@ extern "C" int rn_gsu_fwd(const int32_t *idx, const float *val, const int64_t *i
     p.mask = mask;
     if (mask) { p.mb = mask_strides[0]; p.mt = mask_strides[1]; }
     p.y = y; p.yb = y_strides[0]; p.yh = y_strides[1]; p.yt = y_strides[2];
-    p.slot_in = slot_in; p.slot_out = slot_out; p.mass_in = mass_in; p.mass_out = mass_out;
+    p.slot_in = slot_in; p.slot_out = slot_out; p.mass_in = mass_in; p.mass_out = mass_out; p.mass_init = float(mass_init);
     p.B = int(B); p.H = int(H); p.T = int(T); p.A = int(A); p.C = int(C); p.Kw = int(Kw); p.Kr = int(Kr);
     p.L = pl.L; p.nchunks = pl.nchunks; p.NE = pl.NE; p.NEp = pl.NEp;
     p.row_shift = rn_row_shift(A);
@@ -955,9 +968,11 @@ extern "C" int rn_gsu_fwd(const int32_t *idx, const float *val, const int64_t *i
                          ((x_strides[0] | x_strides[1] | x_strides[2] | y_strides[0] | y_strides[1] | y_strides[2]) & 3) == 0;
     const bool fast = pl.fast && aligned;
 
-    if (!pl.state_in_smem && slot_in != slot_out)
+    if (!pl.state_in_smem && slot_in == nullptr)
+        RN_CUDA(cudaMemsetAsync(slot_out, 0, size_t(B * H * A * C) * 4, stream));
+    else if (!pl.state_in_smem && slot_in != slot_out)
         RN_CUDA(cudaMemcpyAsync(slot_out, slot_in, size_t(B * H * A * C) * 4, cudaMemcpyDeviceToDevice, stream));
-    if (!pl.smem_tables && mass_in != mass_out)
+    if (!pl.smem_tables && mass_in != nullptr && mass_in != mass_out)
         RN_CUDA(cudaMemcpyAsync(mass_out, mass_in, size_t(B * H * A) * 4, cudaMemcpyDeviceToDevice, stream));
 
     if (dtype == RN_F32) return rn_launch_gsu<float>(p, pl, fast, stream);

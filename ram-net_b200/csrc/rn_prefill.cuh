@@ -99,6 +99,7 @@ struct RnGsuParams {
     float *slot_out;
     const float *mass_in;
     float *mass_out;
+    float mass_init;          // mass of every slot when mass_in is null; a null slot_in stands for rows of zeros
     int B, H, T, A, C, Kw, Kr, L, nchunks, NE, NEp;
     int mass_aware;
     float eps;

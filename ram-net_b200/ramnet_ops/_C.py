@@ -22,6 +22,8 @@ if not _LIB_PATH.exists():
 
 lib = ctypes.CDLL(str(_LIB_PATH))
 
+from . import _host as host  # noqa: E402  native host path of the public calls (built together with the library)
+
 _i64, _i32, _f64, _ptr = ctypes.c_int64, ctypes.c_int, ctypes.c_double, ctypes.c_void_p
 _i64p = ctypes.POINTER(ctypes.c_int64)
 

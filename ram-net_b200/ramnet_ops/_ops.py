@@ -70,32 +70,20 @@ def _require_cuda(*tensors: torch.Tensor) -> None:
             raise RuntimeError("ramnet_ops CUDA operators need CUDA tensors")
 
 
-_WORKSPACES: dict[tuple[int, int], torch.Tensor] = {}
-
-
 def _workspace(like: torch.Tensor, nbytes: int) -> torch.Tensor:
     """Scratch for one kernel sequence on the current stream of ``like.device``.
 
     One buffer per (device, stream) is kept and grown on demand, so steady-state calls allocate nothing (a
     fresh gigabyte-sized block per call can make the caching allocator go back to the driver).  Calls on one
-    stream are ordered, so they may share it; every call rewrites what it later reads.  During a stream
-    capture the buffer comes from the capturing allocator instead and is not kept."""
-    nbytes = max(int(nbytes), 256)
-    if torch.cuda.is_current_stream_capturing():
-        return torch.empty(nbytes, dtype=torch.uint8, device=like.device)
-    key = (like.device.index, torch.cuda.current_stream(like.device).cuda_stream)
-    ws = _WORKSPACES.get(key)
-    if ws is None or ws.numel() < nbytes:
-        _WORKSPACES.pop(key, None)
-        ws = None
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=like.device)
-        _WORKSPACES[key] = ws
-    return ws
+    stream are ordered, so they may share it (and with the calls of the native host path, whose table this is);
+    every call rewrites what it later reads.  During a stream capture the buffer comes from the capturing
+    allocator instead and is not kept."""
+    return _C.host.workspace(like.device.index, torch.cuda.current_stream(like.device).cuda_stream, int(nbytes))
 
 
 def release_workspaces() -> None:
     """Drop the cached scratch buffers (they are re-created on the next call)."""
-    _WORKSPACES.clear()
+    _C.host.release_workspaces()
 
 
 def _int32(t: torch.Tensor) -> torch.Tensor:

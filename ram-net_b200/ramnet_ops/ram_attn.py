@@ -18,16 +18,25 @@ from .impl.torch_impl import _torch_ram_attn, _torch_topk_addr
 _triton_ram_attn = None
 _cuda_load_error: Exception | None = None
 try:
+    from . import _C
     from .impl.cuda_impl import _cuda_ram_attn, _cuda_topk_addr
 except Exception as exc:  # pragma: no cover - exercised only without the built library
     _cuda_load_error = exc
     warnings.warn(f"Failed to load the CUDA implementation: {exc}. Build it with `python ram-net_b200/build.py`.")
+    _C = None
     _cuda_ram_attn = None
     _cuda_topk_addr = None
 
 ImplCallableType = Callable[..., tuple[torch.Tensor, torch.Tensor, torch.Tensor]]
 
 _CUDA_DTYPES = (torch.float16, torch.bfloat16, torch.float32)
+
+
+def _native() -> bool:
+    """Whether a call may go through the native host path (csrc/host/rn_host.cpp), which takes the plain form of a call
+    and declines everything else: not under a compiler, which has to see the registered operators, and not in the
+    mode that checks the device status after every operator."""
+    return _C is not None and not torch.compiler.is_compiling() and not _C.CHECK_STATUS
 
 
 def get_broadcast(*vals: int) -> int:
@@ -60,6 +69,11 @@ def topk_addr(
     :return: ``(idx, val)``, both (B, H, K, T); int32 indices and float32 weights.  Entry k is
         the k-th address under (score descending, content index ascending).
     """
+    if _native():
+        out = _C.host.topk_addr(addr, embed_num, position_ids, top_k, top_k_re_norm, addr_val_neg, encode_batch_idx) \
+            if impl_backend is None or impl_backend == 'cuda' else None
+        if out is not None:
+            return out
     assert isinstance(addr, torch.Tensor), f"Expected addr to be Tensor, got {type(addr).__name__}."
     if not isinstance(top_k_re_norm, (int, float)):
         raise TypeError("`top_k_re_norm` must be a number in [0, 1].")
@@ -132,6 +146,11 @@ def random_access_memory_attention(
     :param impl_backend: 'torch', 'cuda' ('triton' is accepted for API parity but not provided) or None.
     :return: ``(output, (slot, mass))`` shaped like values, (..., H, P**U, C) and (..., H, P**U).
     """
+    if _native():
+        out = _C.host.attention(w_addr, r_addr, values, gamma, init_ram, mask, embed_num, position_ids, top_k, top_k_re_norm,
+                                mass_aware, eps, t_dim, inplace, impl_backend)
+        if out is not None:
+            return out
     assert all(isinstance(v, torch.Tensor) for v in (r_addr, w_addr, values)), \
         f"Expected r_addr/w_addr/values to be tensors, got {type(r_addr).__name__}, {type(w_addr).__name__}, {type(values).__name__}."
     if init_ram is None:
