@@ -110,6 +110,10 @@ template <typename T> __device__ __forceinline__ RnRaw4<T> rn_zero_raw4() { RnRa
 template <> __device__ __forceinline__ RnRaw4<float> rn_zero_raw4<float>() { RnRaw4<float> r; r.v = make_float4(0.f, 0.f, 0.f, 0.f); return r; }
 template <typename T> __device__ __forceinline__ RnRaw4<T> rn_load_raw4(const T *p) { RnRaw4<T> r; r.v = *reinterpret_cast<const uint2 *>(p); return r; }
 template <> __device__ __forceinline__ RnRaw4<float> rn_load_raw4<float>(const float *p) { RnRaw4<float> r; r.v = *reinterpret_cast<const float4 *>(p); return r; }
+// pins the first use of a prefetched value to this place: without it the conversion may be moved up to the load, which
+// turns the prefetch into a wait
+__device__ __forceinline__ void rn_pin(RnRaw4<float> &r) { asm volatile("" : "+f"(r.v.x), "+f"(r.v.y), "+f"(r.v.z), "+f"(r.v.w)); }
+template <typename T> __device__ __forceinline__ void rn_pin(RnRaw4<T> &r) { asm volatile("" : "+r"(r.v.x), "+r"(r.v.y)); }
 __device__ __forceinline__ float4 rn_cvt_raw4(const RnRaw4<float> &r) { return r.v; }
 __device__ __forceinline__ float4 rn_cvt_raw4(const RnRaw4<__half> &r) {
     const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&r.v.x));

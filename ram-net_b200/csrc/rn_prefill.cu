@@ -3,7 +3,7 @@
 // (packages/ramnet-ops/src/ramnet_ops/impl/cuda_impl.py:72-141,
 //  packages/ramnet-ops/csrc/ram_attn_segment_parallel.cu:241-416): no global sort, no
 // per-event atomics into y, y written once in the I/O dtype.
-#include "rn_prefill.cuh"
+#include "rn_lists.cuh"
 
 // ------------------------------------------------------------------------------------------
 // schedule kernel: EPT events per thread live in registers across all phases of a chunk
@@ -420,243 +420,6 @@ __global__ void __launch_bounds__(RN_GSU_THREADS) rn_gsu_apply_kernel(const RnGs
 }
 
 // ------------------------------------------------------------------------------------------
-// fast apply kernel: C % 4 == 0, A <= 65536; slice state + streamed chunk records in shared memory.
-//
-// The first event of every slot in a chunk (~80 % of the events) is applied token-major: the CTA's
-// threads are split into one group per token; thread (q, sub) of a group owns the events k = q,
-// q + KL, ... of that token for the 4 channels sub*4 .. sub*4+3, with x[t] in registers and the
-// token's output accumulating in registers.  First events touch pairwise different slots, so a
-// thread requests the records and then the rows of all its events before it uses any of them.
-// The later events of a slot form a chain (link words of the record); the chains of a chunk are
-// dealt evenly to the thread groups from the record's head list, a group walks its chain with the
-// row in registers, and the reads of a chain go through a per-(token,k) buffer to the token's
-// owners.  Two CTA barriers per chunk; the records are double buffered by 1-D bulk copies and only
-// one thread polls the copy's mbarrier.
-// ------------------------------------------------------------------------------------------
-// MODEL: the instance for Kw = Kr = 16 with 64-token chunks (2048 events, 16 threads per token): these are then
-// compile-time constants, so the index arithmetic of the event loops folds into shifts.
-template <typename T, int CS, int EV, bool MODEL = false>
-__global__ void __launch_bounds__(RN_APPLY_THREADS, 1) rn_gsu_apply_fast_kernel(const RnGsuParams p, const int tpt_log2_) {
-    constexpr int G = CS / 4;  // threads per event (one float4 of channels each)
-    extern __shared__ __align__(16) unsigned char dyn[];
-    __shared__ __align__(8) uint64_t mbar[2];
-
-    const int slice = blockIdx.x % p.nslices;
-    const int bh = blockIdx.x / p.nslices;
-    const int b = bh / p.H, h = bh % p.H;
-    const int tid = threadIdx.x;
-    const int C = p.C, A = p.A;
-    const int Kw = MODEL ? 16 : p.Kw, Kr = MODEL ? 16 : p.Kr, KT = MODEL ? 32 : p.Kw + p.Kr, L = MODEL ? 64 : p.L;
-    const int NEp = MODEL ? 2048 : p.NEp;
-    const int tpt_log2 = MODEL ? 4 : tpt_log2_;
-    const int c0 = slice * CS;
-    const int cvalid = min(CS, C - c0);  // multiple of 4
-    const uint32_t rec_copy = uint32_t(size_t(NEp) * 9 + 16);  // {coef, link}[NEp], heads[8 + NEp/2]
-    const uint32_t kt_magic = 0xffffffffu / uint32_t(KT) + 1u;  // e / KT == __umulhi(e, kt_magic) for e < 4096
-
-    // thread -> (token of the chunk, k-lane, channel group)
-    const int TPT = 1 << tpt_log2;          // threads per token (8, 16 or 32: a group never leaves its warp)
-    const int KL = TPT / G;                 // k-lanes per token
-    const int tok = tid >> tpt_log2;        // tokens >= L (surplus threads) take no token-major work
-    const int w = tid & (TPT - 1);
-    const int sub = w % G, q = w / G;
-    const bool chan_ok = MODEL || sub * 4 < cvalid;  // MODEL: C is a multiple of the slice width
-    // is this thread's j-th event a write?  MODEL: 8 k-lanes per token, so events 0, 1 are writes and 2, 3 reads
-    auto wr_of = [&](int j) { return MODEL ? (j < 2) : (q + j * KL < Kw); };
-
-    // dynamic smem: rec[2][rec_stride] | S[A*CS] | xt[L*CS] | ylate[L*Kr*CS]
-    const size_t rec_stride = (size_t(rec_copy) + 127) / 128 * 128;
-    unsigned char *rec0 = dyn;
-    float *S = reinterpret_cast<float *>(dyn + 2 * rec_stride);
-    float *xt = S + size_t(A) * CS;
-    float *ylate = xt + size_t(L) * CS;
-
-    if (tid == 0) {
-        rn_mbar_init(&mbar[0], 1);
-        rn_mbar_init(&mbar[1], 1);
-        rn_mbar_fence_init();
-    }
-    __syncthreads();
-    // the part of a chunk record this kernel reads: the {coef, link} pairs and the head list, contiguous
-    const unsigned char *records = p.records + int64_t(bh) * p.nchunks * p.rec_bytes + RN_GSU_HDR_BYTES + size_t(NEp) * 8;
-    auto fetch = [&](int chunk) {  // one thread; the target buffer was last read before a CTA barrier
-        uint64_t *bar = &mbar[chunk & 1];
-        rn_mbar_expect_tx(bar, rec_copy);
-        rn_bulk_g2s(rec0 + (chunk & 1) * rec_stride, records + int64_t(chunk) * p.rec_bytes, rec_copy, bar);
-    };
-    auto landed = [&](int chunk) {  // one thread: bounded wait for the copy of a chunk's record
-        return rn_mbar_wait_bounded(&mbar[chunk & 1], uint32_t(chunk >> 1) & 1u);
-    };
-    bool failed = false;
-    if (tid == 0) fetch(0);
-
-    // state slice -> shared memory
-    {
-        const float *src = p.slot_in ? p.slot_in + int64_t(bh) * A * C + c0 : nullptr;
-        for (int i = tid; i < A * G; i += RN_APPLY_THREADS) {
-            const int a = i / G, sg = i - a * G;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (src != nullptr && sg * 4 < cvalid) v = *reinterpret_cast<const float4 *>(src + int64_t(a) * C + sg * 4);
-            *reinterpret_cast<float4 *>(S + rn_row_of_slot(uint32_t(a), A, p.row_shift) * CS + sg * 4) = v;
-        }
-    }
-    const T *x = static_cast<const T *>(p.x) + b * p.xb + h * p.xh + c0 + sub * 4;
-    T *y = static_cast<T *>(p.y) + b * p.yb + h * p.yh + c0 + sub * 4;
-
-    auto load_x = [&](int chunk) {  // raw bits: converted one chunk later, when the load has long landed
-        const int t = chunk * L + tok;
-        RnRaw4<T> v = rn_zero_raw4<T>();
-        if (chunk < p.nchunks && tok < L && t < p.T && chan_ok) v = rn_load_raw4<T>(x + int64_t(t) * p.xt);
-        return v;
-    };
-
-    RnRaw4<T> xnext = load_x(0);
-    if (tid == 0 && !landed(0)) failed = true;
-    if (__syncthreads_or(failed)) {  // state and barriers are set up, the first record has landed
-        if (tid == 0) atomicMax(p.status, RN_STATUS_WAIT_TIMEOUT);
-        return;
-    }
-
-    for (int chunk = 0; chunk < p.nchunks; ++chunk) {
-        const int t0 = chunk * L;
-        const bool tok_ok = tok < min(L, p.T - t0);
-        const bool has_next = chunk + 1 < p.nchunks;
-        const float4 xv = rn_cvt_raw4(xnext);
-        if (tid == 0 && has_next) fetch(chunk + 1);
-        xnext = load_x(chunk + 1);
-        const unsigned char *rec = rec0 + (chunk & 1) * rec_stride;
-        const uint2 *e_pair = reinterpret_cast<const uint2 *>(rec);
-        const uint16_t *heads = reinterpret_cast<const uint16_t *>(rec + size_t(NEp) * 8);
-
-        // ---- first events, token-major: records, then rows, then arithmetic, then stores ------------------
-        if (q == 0 && tok < L) *reinterpret_cast<float4 *>(xt + tok * CS + sub * 4) = xv;
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        uint32_t late = 0;  // this thread's reads that a chain delivers
-        constexpr int NB = EV < 2 ? EV : 2;  // events in flight per thread
-#pragma unroll
-        for (int jb = 0; jb < EV; jb += NB) {
-            uint2 pr[NB];
-            float4 row[NB];
-#pragma unroll
-            for (int i = 0; i < NB; ++i) {
-                const int k = q + (jb + i) * KL;
-                pr[i] = make_uint2(0u, RN_LINK_DEAD);
-                if (tok_ok && (MODEL || k < KT)) pr[i] = e_pair[tok * KT + k];
-            }
-#pragma unroll
-            for (int i = 0; i < NB; ++i) {
-                const uint32_t kind = (pr[i].y >> RN_LINK_KIND_SHIFT) & 7u;  // bit 2: dead
-                if (kind < RN_KIND_HEAD) {
-                    row[i] = *reinterpret_cast<const float4 *>(S + (pr[i].y & 0xffffu) * CS + sub * 4);
-                } else if (kind <= RN_KIND_LATER && !wr_of(jb + i)) {
-                    late |= 1u << (jb + i);
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < NB; ++i) {
-                if (((pr[i].y >> RN_LINK_KIND_SHIFT) & 7u) >= RN_KIND_HEAD) continue;
-                const float cf = __uint_as_float(pr[i].x);
-                if (wr_of(jb + i)) {
-                    float4 s = row[i];
-                    s.x = fmaf(cf, xv.x - s.x, s.x);
-                    s.y = fmaf(cf, xv.y - s.y, s.y);
-                    s.z = fmaf(cf, xv.z - s.z, s.z);
-                    s.w = fmaf(cf, xv.w - s.w, s.w);
-                    *reinterpret_cast<float4 *>(S + (pr[i].y & 0xffffu) * CS + sub * 4) = s;
-                } else {
-                    acc.x = fmaf(cf, row[i].x, acc.x);
-                    acc.y = fmaf(cf, row[i].y, acc.y);
-                    acc.z = fmaf(cf, row[i].z, acc.z);
-                    acc.w = fmaf(cf, row[i].w, acc.w);
-                }
-            }
-        }
-        __syncthreads();
-
-        // ---- the chains of this chunk, dealt to the thread groups ----------------------------------------
-        {
-            const int n_heads = heads[0];
-            const int csub = tid % G;
-            for (int i = tid / G; i < n_heads; i += RN_APPLY_THREADS / G) {
-                int e = heads[8 + i];
-                uint2 pr = e_pair[e];
-                float *row = S + (pr.y & 0xffffu) * CS + csub * 4;
-                float4 s = *reinterpret_cast<float4 *>(row);
-                bool dirty = false;
-                for (int guard = 0; guard < RN_GSU_NE_MAX; ++guard) {
-                    // the following event's record is requested before this one is applied
-                    const bool more = (pr.y & RN_LINK_NEXT) != 0;
-                    const int en = int((pr.y >> 16) & 0xfffu);
-                    uint2 pr_n = make_uint2(0u, 0u);
-                    if (more) pr_n = e_pair[en];
-                    const float cf = __uint_as_float(pr.x);
-                    const int ct = int(__umulhi(uint32_t(e), kt_magic)), ck = e - ct * KT;
-                    // one instruction stream for writes and reads: the lanes of a warp hold both kinds
-                    const bool wr = ck < Kw;
-                    const float4 xr = *reinterpret_cast<const float4 *>(xt + ct * CS + csub * 4);
-                    if (!wr)
-                        *reinterpret_cast<float4 *>(ylate + (ct * Kr + (ck - Kw)) * CS + csub * 4) =
-                            make_float4(cf * s.x, cf * s.y, cf * s.z, cf * s.w);
-                    const float g = wr ? cf : 0.f;  // a read leaves the row as it is
-                    s.x = fmaf(g, xr.x - s.x, s.x);
-                    s.y = fmaf(g, xr.y - s.y, s.y);
-                    s.z = fmaf(g, xr.z - s.z, s.z);
-                    s.w = fmaf(g, xr.w - s.w, s.w);
-                    dirty |= wr;
-                    if (!more) break;
-                    e = en;
-                    pr = pr_n;
-                }
-                if (dirty) *reinterpret_cast<float4 *>(row) = s;
-            }
-        }
-        // the next record (requested at the top of this step) has to be there for the next step
-        if (tid == 0 && has_next && !landed(chunk + 1)) failed = true;
-        if (__syncthreads_or(failed)) {
-            if (tid == 0) atomicMax(p.status, RN_STATUS_WAIT_TIMEOUT);
-            return;
-        }
-
-        // ---- reads delivered by the chains, then combine the k-lanes ----------------------------------------
-#pragma unroll
-        for (int j = 0; j < EV; ++j) {
-            if (!(late & (1u << j))) continue;
-            const int k = q + j * KL;
-            const float4 v = *reinterpret_cast<const float4 *>(ylate + (tok * Kr + (k - Kw)) * CS + sub * 4);
-            acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-        }
-        if (KL >= 4) {
-            // transposing butterfly over the k-lanes: after two exchange levels lane (q & 3) holds one channel
-            const bool b0 = (q & 1) != 0, b1 = (q & 2) != 0;
-            float k0 = b0 ? acc.z : acc.x, k1 = b0 ? acc.w : acc.y;
-            const float s0 = b0 ? acc.x : acc.z, s1 = b0 ? acc.y : acc.w;
-            k0 += __shfl_xor_sync(RN_FULL, s0, G);
-            k1 += __shfl_xor_sync(RN_FULL, s1, G);
-            float r = b1 ? k1 : k0;
-            r += __shfl_xor_sync(RN_FULL, b1 ? k0 : k1, 2 * G);
-            for (int off = 4 * G; off < TPT; off <<= 1) r += __shfl_xor_sync(RN_FULL, r, off);
-            if (q < 4 && tok_ok && chan_ok) y[int64_t(t0 + tok) * p.yt + (b0 ? 2 : 0) + (b1 ? 1 : 0)] = rn_from_float<T>(r);
-        } else {
-            for (int off = G; off < TPT; off <<= 1) {
-                acc.x += __shfl_xor_sync(RN_FULL, acc.x, off);
-                acc.y += __shfl_xor_sync(RN_FULL, acc.y, off);
-                acc.z += __shfl_xor_sync(RN_FULL, acc.z, off);
-                acc.w += __shfl_xor_sync(RN_FULL, acc.w, off);
-            }
-            if (q == 0 && tok_ok && chan_ok) rn_store4<T>(y + int64_t(t0 + tok) * p.yt, acc);
-        }
-    }
-
-    __syncthreads();
-    float *dst = p.slot_out + int64_t(bh) * A * C + c0;
-    for (int i = tid; i < A * G; i += RN_APPLY_THREADS) {
-        const int a = i / G, sg = i - a * G;
-        if (sg * 4 < cvalid)
-            *reinterpret_cast<float4 *>(dst + int64_t(a) * C + sg * 4) = *reinterpret_cast<const float4 *>(S + rn_row_of_slot(uint32_t(a), A, p.row_shift) * CS + sg * 4);
-    }
-}
-
-// ------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------
 constexpr size_t RN_SMEM_BUDGET = 225 * 1024;
@@ -762,7 +525,9 @@ extern "C" int64_t rn_gsu_workspace_bytes(int64_t B, int64_t H, int64_t T, int64
     rn_clear_error();
     RnGsuPlan pl;
     if (rn_gsu_plan(B, H, T, A, C, Kw, Kr, device, &pl)) return -1;
-    return int64_t(pl.total);
+    RnListPlan lp;
+    const size_t lists = rn_list_plan(B, H, T, A, C, Kw, Kr, 1, &lp) ? lp.total : 0;
+    return int64_t(pl.total > lists ? pl.total : lists);
 }
 
 // Which kernels a prefill call of this shape runs, for tests and benchmarks that must prove they exercise the
@@ -793,10 +558,10 @@ extern "C" int64_t rn_gsu_fwd_workspace_bytes(int dtype, int rows_aligned, int64
             rn_gsu_owner_clusters(dtype, device) > 0)
             return 0;
     }
-    return int64_t(pl.total);
+    return rn_gsu_workspace_bytes(B, H, T, A, C, Kw, Kr, device);
 }
 
-// Which forward path rn_gsu_fwd takes for a shape: 0 general apply kernel, 1 channel-slice kernels with per-slot chains,
+// Which forward path rn_gsu_fwd takes for a shape: 0 general apply kernel, 1 event-list kernels (rn_lists.cuh),
 // 2 slot-owner cluster kernel.  rows_aligned: x / y rows start on 16-byte boundaries.
 extern "C" int rn_gsu_fwd_path(int dtype, int rows_aligned, int64_t B, int64_t H, int64_t T, int64_t A, int64_t C, int64_t Kw,
                                int64_t Kr, int device) {
@@ -804,7 +569,8 @@ extern "C" int rn_gsu_fwd_path(int dtype, int rows_aligned, int64_t B, int64_t H
     RnGsuPlan pl;
     if (rn_gsu_plan(B, H, T, A, C, Kw, Kr, device, &pl)) return -1;
     if (rn_gsu_fwd_workspace_bytes(dtype, rows_aligned, B, H, T, A, C, Kw, Kr, device) == 0) return 2;
-    return (pl.fast && rows_aligned) ? 1 : 0;
+    RnListPlan lp;
+    return rows_aligned && rn_list_plan(B, H, T, A, C, Kw, Kr, 0, &lp) ? 1 : 0;
 }
 
 template <typename T, bool SMEM>
@@ -823,30 +589,6 @@ static int rn_launch_schedule(const RnGsuParams &p, const RnGsuPlan &pl, cudaStr
     return 1;
 }
 
-template <typename T>
-static int rn_launch_apply_fast(const RnGsuParams &p, const RnGsuPlan &pl, cudaStream_t stream) {
-    const int grid = p.B * p.H * pl.nslices;
-    if (pl.cs == 8 && pl.ev == 4 && p.Kw == 16 && p.Kr == 16 && pl.L == 64 && pl.NEp == 2048 && pl.tpt_log2 == 4 && p.C % 8 == 0) {
-        RN_CUDA(cudaFuncSetAttribute(rn_gsu_apply_fast_kernel<T, 8, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(pl.apply_smem)));
-        rn_gsu_apply_fast_kernel<T, 8, 4, true><<<grid, RN_APPLY_THREADS, pl.apply_smem, stream>>>(p, pl.tpt_log2);
-        return 0;
-    }
-#define RN_CASE(CSV, EVV)                                                                                       \
-    if (pl.cs == CSV && pl.ev == EVV) {                                                                         \
-        RN_CUDA(cudaFuncSetAttribute(rn_gsu_apply_fast_kernel<T, CSV, EVV>,                                     \
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, int(pl.apply_smem)));         \
-        rn_gsu_apply_fast_kernel<T, CSV, EVV><<<grid, RN_APPLY_THREADS, pl.apply_smem, stream>>>(p, pl.tpt_log2); \
-        return 0;                                                                                               \
-    }
-#define RN_CASES(CSV) RN_CASE(CSV, 1) RN_CASE(CSV, 2) RN_CASE(CSV, 4) RN_CASE(CSV, 8) RN_CASE(CSV, 16)
-    RN_CASES(4) RN_CASES(8) RN_CASES(16) RN_CASES(32)
-#undef RN_CASES
-#undef RN_CASE
-    rn_set_error("no fast apply kernel for %d channels per CTA, %d events per thread", pl.cs, pl.ev);
-    return 1;
-}
-
 int rn_gsu_launch_schedule(const RnGsuParams &p, const RnGsuPlan &pl, int dtype, cudaStream_t stream) {
     if (dtype == RN_F32)
         return pl.smem_tables ? rn_launch_schedule<float, true>(p, pl, stream) : rn_launch_schedule<float, false>(p, pl, stream);
@@ -857,20 +599,15 @@ int rn_gsu_launch_schedule(const RnGsuParams &p, const RnGsuPlan &pl, int dtype,
 }
 
 template <typename T>
-static int rn_launch_gsu(const RnGsuParams &p, const RnGsuPlan &pl, bool fast, cudaStream_t stream) {
+static int rn_launch_gsu(const RnGsuParams &p, const RnGsuPlan &pl, cudaStream_t stream) {
     rn_prof_reset();
     rn_prof_mark(stream);
     if (int rc = pl.smem_tables ? rn_launch_schedule<T, true>(p, pl, stream) : rn_launch_schedule<T, false>(p, pl, stream))
         return rc;
     RN_CUDA(cudaGetLastError());
     rn_prof_mark(stream);
-    if (fast) {
-        if (int rc = rn_launch_apply_fast<T>(p, pl, stream)) return rc;
-    } else {
-        RN_CUDA(cudaFuncSetAttribute(rn_gsu_apply_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(pl.apply_smem)));
-        rn_gsu_apply_kernel<T><<<p.B * p.H * pl.nslices, RN_GSU_THREADS, pl.apply_smem, stream>>>(p);
-    }
+    RN_CUDA(cudaFuncSetAttribute(rn_gsu_apply_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(pl.apply_smem)));
+    rn_gsu_apply_kernel<T><<<p.B * p.H * pl.nslices, RN_GSU_THREADS, pl.apply_smem, stream>>>(p);
     RN_CUDA(cudaGetLastError());
     rn_prof_mark(stream);
     return 0;
@@ -936,6 +673,42 @@ extern "C" int rn_gsu_fwd_init(const int32_t *idx, const float *val, const int64
         if (rc > 0) return rc;
         // rc < 0: this device cannot keep a 16-CTA cluster of that size resident; use the channel-slice kernels
     }
+    const size_t esz = dtype == RN_F32 ? 4 : 2;
+    // the list kernels and the fast apply kernel move x / y in 4-element vectors
+    const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & (4 * esz - 1)) == 0 &&
+                         ((x_strides[0] | x_strides[1] | x_strides[2] | y_strides[0] | y_strides[1] | y_strides[2]) & 3) == 0;
+    RnListPlan lp;
+    if (aligned && rn_list_plan(B, H, T, A, C, Kw, Kr, mass_aware, &lp)) {
+        RN_REQUIRE(workspace != nullptr && workspace_bytes >= int64_t(lp.total), "workspace too small: %lld < %lld bytes",
+                   (long long)workspace_bytes, (long long)lp.total);
+        RN_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "workspace must be 256-byte aligned");
+        RnListParams q{};
+        q.idx = idx; q.val = val;
+        q.ib = idx_strides[0]; q.ih = idx_strides[1]; q.ik = idx_strides[2]; q.it = idx_strides[3];
+        q.gamma = gamma; q.gb = gamma_strides[0]; q.gh = gamma_strides[1]; q.gt = gamma_strides[2];
+        q.mask = mask;
+        if (mask) { q.mb = mask_strides[0]; q.mt = mask_strides[1]; }
+        q.x = x; q.xb = x_strides[0]; q.xh = x_strides[1]; q.xt = x_strides[2];
+        q.y = y; q.yb = y_strides[0]; q.yh = y_strides[1]; q.yt = y_strides[2];
+        q.slot_in = slot_in; q.slot_out = slot_out; q.mass_in = mass_in; q.mass_out = mass_out; q.mass_init = float(mass_init);
+        q.B = int(B); q.H = int(H); q.T = int(T); q.A = int(A); q.C = int(C); q.Kw = int(Kw); q.Kr = int(Kr);
+        q.L = lp.L; q.nblocks = lp.nblocks; q.lg = lp.lg; q.lr = lp.lr; q.ngroups = lp.ngroups; q.capR = lp.capR; q.capW = lp.capW;
+        q.blk_bytes = lp.blk_bytes; q.list_max = lp.list_max; q.whole_max = lp.whole_max; q.step_max = lp.step_max;
+        q.rs = lp.cs == 32 ? 7 : 6;
+        q.a_magic = 0xffffffffu / uint32_t(A);
+        q.mass_aware = mass_aware; q.eps = float(eps);
+        q.status = rn_status_word(device);
+        RN_REQUIRE(q.status != nullptr, "cannot locate the status word of device %d", device);
+        q.recs = static_cast<unsigned char *>(workspace);
+        q.first = reinterpret_cast<uint4 *>(q.recs + lp.off_first);
+        rn_prof_reset();
+        rn_prof_mark(stream);
+        if (int rc = rn_launch_lists(q, lp, dtype, stream)) return rc;
+        if (int rc = rn_launch_apply(q, lp, dtype, stream)) return rc;
+        RN_CUDA(cudaGetLastError());
+        rn_prof_mark(stream);
+        return 0;
+    }
     RN_REQUIRE(workspace != nullptr && workspace_bytes >= int64_t(pl.total), "workspace too small: %lld < %lld bytes",
                (long long)workspace_bytes, (long long)pl.total);
     RN_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "workspace must be 256-byte aligned");
@@ -962,12 +735,6 @@ extern "C" int rn_gsu_fwd_init(const int32_t *idx, const float *val, const int64
     p.claim = reinterpret_cast<uint32_t *>(ws + pl.off_claim);
     p.cs = pl.cs; p.nslices = pl.nslices; p.state_in_smem = pl.state_in_smem;
 
-    // the fast apply kernel moves x / y in 4-element vectors
-    const size_t esz = dtype == RN_F32 ? 4 : 2;
-    const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & (4 * esz - 1)) == 0 &&
-                         ((x_strides[0] | x_strides[1] | x_strides[2] | y_strides[0] | y_strides[1] | y_strides[2]) & 3) == 0;
-    const bool fast = pl.fast && aligned;
-
     if (!pl.state_in_smem && slot_in == nullptr)
         RN_CUDA(cudaMemsetAsync(slot_out, 0, size_t(B * H * A * C) * 4, stream));
     else if (!pl.state_in_smem && slot_in != slot_out)
@@ -975,9 +742,9 @@ extern "C" int rn_gsu_fwd_init(const int32_t *idx, const float *val, const int64
     if (!pl.smem_tables && mass_in != nullptr && mass_in != mass_out)
         RN_CUDA(cudaMemcpyAsync(mass_out, mass_in, size_t(B * H * A) * 4, cudaMemcpyDeviceToDevice, stream));
 
-    if (dtype == RN_F32) return rn_launch_gsu<float>(p, pl, fast, stream);
-    if (dtype == RN_F16) return rn_launch_gsu<__half>(p, pl, fast, stream);
-    return rn_launch_gsu<__nv_bfloat16>(p, pl, fast, stream);
+    if (dtype == RN_F32) return rn_launch_gsu<float>(p, pl, stream);
+    if (dtype == RN_F16) return rn_launch_gsu<__half>(p, pl, stream);
+    return rn_launch_gsu<__nv_bfloat16>(p, pl, stream);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1034,7 +801,36 @@ extern "C" int rn_gsu_fwd_static(const int32_t *idx, const float *val, const int
         RN_REQUIRE(guard.ok, "cannot make device %d current", device);
         if (int rc = rn_static_scratch_ptr(device, &scratch)) return rc;
     }
-    return rn_gsu_fwd(idx, val, idx_strides, x, x_strides, gamma, gamma_strides, dtype, mask, mask_strides, slot_in,
-                      mass_in, slot_out, mass_out, y, y_strides, scratch, int64_t(RN_STATIC_SCRATCH_BYTES), B, H, T, A, C,
-                      Kw, Kr, mass_aware, eps, device, stream);
+    RN_REQUIRE(idx && val && idx_strides && x && x_strides && gamma && gamma_strides && slot_in && mass_in && slot_out && mass_out &&
+                   y && y_strides && (mask == nullptr || mask_strides != nullptr) && dtype >= RN_F32 && dtype <= RN_BF16,
+               "null pointer argument");
+    // The event lists of a long sequence may be larger than the array although the bound above holds: the call then runs in
+    // pieces, shorter in time (the state carries over) or, if one block of all heads does not fit, head by head.
+    const size_t esz = dtype == RN_F32 ? 4 : 2;
+    int64_t t_piece = T, h_piece = H, b_piece = B;
+    RnListPlan lp;
+    if (rn_list_plan(B, H, T, A, C, Kw, Kr, mass_aware, &lp) && lp.total > RN_STATIC_SCRATCH_BYTES) {
+        const int64_t per_block = lp.blk_bytes + 16 * lp.N, blocks = int64_t(RN_STATIC_SCRATCH_BYTES - 256) / (B * H * per_block);
+        if (blocks > 0) {
+            t_piece = blocks * lp.L;
+        } else {
+            b_piece = h_piece = 1;
+            t_piece = int64_t(RN_STATIC_SCRATCH_BYTES - 256) / per_block * lp.L;
+        }
+    }
+    for (int64_t b = 0; b < B; b += b_piece)
+        for (int64_t h = 0; h < H; h += h_piece)
+            for (int64_t t = 0; t < T; t += t_piece) {
+                const int64_t io = b * idx_strides[0] + h * idx_strides[1] + t * idx_strides[3], so = (b * H + h) * A;
+                auto at = [&](const void *base, const int64_t *s) {
+                    return static_cast<const unsigned char *>(base) + size_t(b * s[0] + h * s[1] + t * s[2]) * esz;
+                };
+                if (int rc = rn_gsu_fwd(idx + io, val + io, idx_strides, at(x, x_strides), x_strides, at(gamma, gamma_strides), gamma_strides,
+                                        dtype, mask ? mask + b * mask_strides[0] + t * mask_strides[1] : nullptr, mask_strides,
+                                        (t ? slot_out : slot_in) + so * C, (t ? mass_out : mass_in) + so, slot_out + so * C, mass_out + so,
+                                        const_cast<unsigned char *>(at(y, y_strides)), y_strides, scratch, int64_t(RN_STATIC_SCRATCH_BYTES),
+                                        b_piece, h_piece, T - t < t_piece ? T - t : t_piece, A, C, Kw, Kr, mass_aware, eps, device, stream))
+                    return rc;
+            }
+    return 0;
 }
