@@ -66,6 +66,10 @@ int launch_fast(const FastParams &p, cudaStream_t stream) {
 template <typename T>
 int dispatch_fast(const FastParams &p, int U, int P, int K, cudaStream_t stream) {
     if (U == 2 && P == 64 && K == 16) return launch_fast<T, 2, 64, 16>(p, stream);
+    if (U == 2 && P == 64 && K == 8) return launch_fast<T, 2, 64, 8>(p, stream);
+    if (U == 2 && P == 64 && K == 32) return launch_fast<T, 2, 64, 32>(p, stream);
+    if (U == 2 && P == 32 && K == 8) return launch_fast<T, 2, 32, 8>(p, stream);
+    if (U == 3 && P == 8 && K == 8) return launch_fast<T, 3, 8, 8>(p, stream);
     if (U == 3 && P == 32 && K == 8) return launch_fast<T, 3, 32, 8>(p, stream);
     if (U == 2 && P == 16 && K == 4) return launch_fast<T, 2, 16, 4>(p, stream);
     if (U == 5 && P == 8 && K == 8) return launch_fast<T, 5, 8, 8>(p, stream);  // 32768 slots at the reference's radix limit
@@ -152,7 +156,7 @@ __global__ void __launch_bounds__(FAST_THREADS) rn_addr_bwd_fast_kernel(const Fa
     constexpr int RPC = FAST_THREADS / LPR; // rows per CTA
     constexpr int EPL = K / LPR;            // Top-K entries per lane
     constexpr int ROW = U * P + (LPR <= 2 ? 4 : 0);  // accumulator stride: short rows are staggered over the banks
-    static_assert(K % LPR == 0 && EPL % 2 == 0, "an even number of Top-K entries per lane");
+    static_assert(K % LPR == 0 && (EPL == 1 || EPL % 2 == 0), "one or an even number of Top-K entries per lane");
     __shared__ __align__(16) float accum[RPC][ROW];
 
     const int tid = threadIdx.x, lr = tid % LPR, rc = tid / LPR;
@@ -175,20 +179,31 @@ __global__ void __launch_bounds__(FAST_THREADS) rn_addr_bwd_fast_kernel(const Fa
     int ce[EPL];
     float we[EPL], de[EPL];
     float dsum = 0.f, wsum = 0.f;
+    int ix[EPL];
+    float wv[EPL], dv[EPL];
+    if constexpr (EPL == 1) {
+        ix[0] = p.idx[o];
+        wv[0] = p.val[o];
+        dv[0] = p.d_val[g];
+    } else {
 #pragma unroll
-    for (int e = 0; e < EPL; e += 2) {
-        const int2 ix = *reinterpret_cast<const int2 *>(p.idx + o + e);
-        const float2 wv = *reinterpret_cast<const float2 *>(p.val + o + e);
-        const float2 dv = *reinterpret_cast<const float2 *>(p.d_val + g + e);
-        we[e] = p.sign[which] * wv.x;
-        we[e + 1] = p.sign[which] * wv.y;
-        de[e] = dv.x * we[e];
-        de[e + 1] = dv.y * we[e + 1];
-        int c0 = ix.x % p.A + shift, c1 = ix.y % p.A + shift;
-        ce[e] = c0 >= p.A ? c0 - p.A : c0;
-        ce[e + 1] = c1 >= p.A ? c1 - p.A : c1;
-        dsum += de[e] + de[e + 1];
-        wsum += we[e] + we[e + 1];
+        for (int e = 0; e < EPL; e += 2) {
+            const int2 i2 = *reinterpret_cast<const int2 *>(p.idx + o + e);
+            const float2 w2 = *reinterpret_cast<const float2 *>(p.val + o + e);
+            const float2 d2 = *reinterpret_cast<const float2 *>(p.d_val + g + e);
+            ix[e] = i2.x; ix[e + 1] = i2.y;
+            wv[e] = w2.x; wv[e + 1] = w2.y;
+            dv[e] = d2.x; dv[e + 1] = d2.y;
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < EPL; ++e) {
+        we[e] = p.sign[which] * wv[e];
+        de[e] = dv[e] * we[e];
+        const int c = ix[e] % p.A + shift;
+        ce[e] = c >= p.A ? c - p.A : c;
+        dsum += de[e];
+        wsum += we[e];
     }
 #pragma unroll
     for (int off = 1; off < LPR; off <<= 1) {
@@ -270,11 +285,20 @@ int launch_bwd_fast(const FastBwdParams &p, cudaStream_t stream) {
 template <typename T>
 int dispatch_bwd_fast(const FastBwdParams &p, int U, int P, int K, cudaStream_t stream) {
     if (U == 2 && P == 64 && K == 16) return launch_bwd_fast<T, 2, 64, 16>(p, stream);
+    if (U == 2 && P == 64 && K == 8) return launch_bwd_fast<T, 2, 64, 8>(p, stream);
+    if (U == 2 && P == 64 && K == 32) return launch_bwd_fast<T, 2, 64, 32>(p, stream);
+    if (U == 2 && P == 32 && K == 8) return launch_bwd_fast<T, 2, 32, 8>(p, stream);
+    if (U == 3 && P == 8 && K == 8) return launch_bwd_fast<T, 3, 8, 8>(p, stream);
     if (U == 3 && P == 32 && K == 8) return launch_bwd_fast<T, 3, 32, 8>(p, stream);
     if (U == 2 && P == 16 && K == 4) return launch_bwd_fast<T, 2, 16, 4>(p, stream);
     if (U == 5 && P == 8 && K == 8) return launch_bwd_fast<T, 5, 8, 8>(p, stream);
     if (U == 4 && P == 8 && K == 16) return launch_bwd_fast<T, 4, 8, 16>(p, stream);
     return -1;
+}
+
+bool has_instance(int64_t U, int64_t P, int64_t K) {
+    return (U == 2 && P == 64 && (K == 8 || K == 16 || K == 32)) || (U == 2 && P == 32 && K == 8) || (U == 2 && P == 16 && K == 4) ||
+           (U == 3 && P == 32 && K == 8) || (U == 3 && P == 8 && K == 8) || (U == 5 && P == 8 && K == 8) || (U == 4 && P == 8 && K == 16);
 }
 
 }  // namespace
@@ -285,9 +309,7 @@ int rn_addr_fwd_fast(const void *w_addr, const void *r_addr, int dtype, const in
                      int64_t H, int64_t U, int64_t P, int64_t T, int64_t E, int64_t A, int64_t Kw, int64_t Kr,
                      double w_re_norm, double r_re_norm, int w_neg, int r_neg, int encode_batch, cudaStream_t stream) {
     if (r_addr != nullptr && Kw != Kr) return -1;
-    const bool shape_ok = (U == 2 && P == 64 && Kw == 16) || (U == 3 && P == 32 && Kw == 8) || (U == 2 && P == 16 && Kw == 4) ||
-                          (U == 5 && P == 8 && Kw == 8) || (U == 4 && P == 8 && Kw == 16);
-    if (!shape_ok) return -1;
+    if (!has_instance(U, P, Kw)) return -1;
     const size_t esz = dtype == RN_F32 ? 4 : 2;
     // the U*P block of a row must be contiguous and 16-byte aligned; the K outputs of a row too
     if (addr_strides[3] != 1 || addr_strides[2] != P) return -1;
@@ -322,9 +344,7 @@ int rn_addr_bwd_fast(const int32_t *idx, const float *val, const int64_t *out_st
                      int64_t A, int64_t Kw, int64_t Kr, double w_re_norm, double r_re_norm, int w_neg, int r_neg,
                      cudaStream_t stream) {
     if (r_addr != nullptr && Kw != Kr) return -1;
-    const bool shape_ok = (U == 2 && P == 64 && Kw == 16) || (U == 3 && P == 32 && Kw == 8) || (U == 2 && P == 16 && Kw == 4) ||
-                          (U == 5 && P == 8 && Kw == 8) || (U == 4 && P == 8 && Kw == 16);
-    if (!shape_ok) return -1;
+    if (!has_instance(U, P, Kw)) return -1;
     const size_t esz = dtype == RN_F32 ? 4 : 2;
     // logits and their gradients: the U*P block of a row contiguous, rows 16-byte aligned (32 for fp32 pairs of float4)
     if (addr_strides[3] != 1 || addr_strides[2] != P || dgrad_strides[3] != 1 || dgrad_strides[2] != P) return -1;

@@ -43,22 +43,26 @@ struct Key64 {
 };
 __device__ __forceinline__ bool key_less(const Key32 &a, const Key32 &b) { return a.v < b.v; }
 __device__ __forceinline__ bool key_less(const Key64 &a, const Key64 &b) {
-    return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo);
+    return ((uint64_t(a.hi) << 32) | a.lo) < ((uint64_t(b.hi) << 32) | b.lo);
 }
 __device__ __forceinline__ void cmpx(Key32 &a, Key32 &b) {  // afterwards a >= b
     const uint32_t mx = max(a.v, b.v), mn = min(a.v, b.v);
     a.v = mx;
     b.v = mn;
 }
+// a comparison and four selects: written as a conditional swap it becomes a branch, which the lanes of a warp take in
+// different ways (a third more instructions at U = 2, P = 64, K = 16)
 __device__ __forceinline__ void cmpx(Key64 &a, Key64 &b) {
-    if (key_less(a, b)) {
-        const Key64 t = a;
-        a = b;
-        b = t;
-    }
+    const bool lt = key_less(a, b);
+    const Key64 t{lt ? b.hi : a.hi, lt ? b.lo : a.lo};
+    b = Key64{lt ? a.hi : b.hi, lt ? a.lo : b.lo};
+    a = t;
 }
 __device__ __forceinline__ Key32 key_max(const Key32 &a, const Key32 &b) { return Key32{max(a.v, b.v)}; }
-__device__ __forceinline__ Key64 key_max(const Key64 &a, const Key64 &b) { return key_less(a, b) ? b : a; }
+__device__ __forceinline__ Key64 key_max(const Key64 &a, const Key64 &b) {
+    const bool lt = key_less(a, b);
+    return Key64{lt ? b.hi : a.hi, lt ? b.lo : a.lo};
+}
 __device__ __forceinline__ Key32 key_lowest(Key32) { return Key32{0u}; }
 __device__ __forceinline__ Key64 key_lowest(Key64) { return Key64{0u, 0u}; }
 
@@ -199,12 +203,19 @@ __device__ __forceinline__ void rn_for_each_logit(const T *src, F &&f) {
             f(4 * v, x.x); f(4 * v + 1, x.y); f(4 * v + 2, x.z); f(4 * v + 3, x.w);
         }
     } else {
+        constexpr int W = P < 8 ? P / 2 : 4;  // words of a vector load
 #pragma unroll
-        for (int v = 0; v < P / 8; ++v) {
-            const uint4 raw = reinterpret_cast<const uint4 *>(src)[v];
-            const uint32_t wds[4] = {raw.x, raw.y, raw.z, raw.w};
+        for (int v = 0; v < (P + 7) / 8; ++v) {
+            uint32_t wds[4];
+            if constexpr (W == 4) {
+                const uint4 raw = reinterpret_cast<const uint4 *>(src)[v];
+                wds[0] = raw.x; wds[1] = raw.y; wds[2] = raw.z; wds[3] = raw.w;
+            } else {
+                const uint2 raw = *reinterpret_cast<const uint2 *>(src);
+                wds[0] = raw.x; wds[1] = raw.y;
+            }
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < W; ++c) {
                 const uint32_t lo = wds[c] & 0xffffu, hi = wds[c] >> 16;
                 if constexpr (std::is_same<T, __nv_bfloat16>::value) {
                     f(8 * v + 2 * c, __uint_as_float(lo << 16));
@@ -218,25 +229,45 @@ __device__ __forceinline__ void rn_for_each_logit(const T *src, F &&f) {
     }
 }
 
-template <typename T, int P>
-__device__ __forceinline__ void rn_make_keys(const T *src, Key64 *dk) {
-    rn_for_each_logit<T, P>(src, [&](int q, float x) { dk[q] = Key64{rn_ord(x + 0.0f), ~uint32_t(q)}; });
+template <typename T> __device__ __forceinline__ uint32_t canonical_zero(uint32_t w);
+template <> __device__ __forceinline__ uint32_t canonical_zero<__nv_bfloat16>(uint32_t w) {
+    uint32_t r;
+    asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(w), "r"(0u));
+    return r;
 }
-template <typename T, int P>
-__device__ __forceinline__ void rn_make_keys(const T *src, Key32 *dk) {
+template <> __device__ __forceinline__ uint32_t canonical_zero<__half>(uint32_t w) {
+    uint32_t r;
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(w), "r"(0u));
+    return r;
+}
+// keys of N consecutive logits, the first of them logit p0 of its digit
+template <typename T, int N>
+__device__ __forceinline__ void rn_make_keys(const T *src, int p0, Key64 *dk) {
+    rn_for_each_logit<T, N>(src, [&](int q, float x) { dk[q] = Key64{rn_ord(x + 0.0f), ~uint32_t(p0 + q)}; });
+}
+template <typename T, int N>
+__device__ __forceinline__ void rn_make_keys(const T *src, int p0, Key32 *dk) {
+    // two logits at a time: -0 made +0 by a packed addition, then all bits flipped below zero and the sign bit above
+    const uint32_t low = 0xffffu - uint32_t(p0);
+    auto pair = [&](uint32_t w, int q) __attribute__((always_inline)) {
+        w = canonical_zero<T>(w);
+        uint32_t sign;
+        asm("prmt.b32 %0, %1, %1, 0xbb99;" : "=r"(sign) : "r"(w));  // the sign of either half, replicated over the half
+        const uint32_t o = w ^ (sign | 0x80008000u);
+        dk[q] = Key32{__byte_perm(o, low - uint32_t(q), 0x1054u)};
+        dk[q + 1] = Key32{__byte_perm(o, low - uint32_t(q + 1), 0x3254u)};
+    };
+    if constexpr (N >= 8) {
 #pragma unroll
-    for (int v = 0; v < P / 8; ++v) {
-        const uint4 raw = reinterpret_cast<const uint4 *>(src)[v];
-        const uint32_t wds[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int q = 8 * v + 2 * c;
-            dk[q] = Key32{(ord16_from_bf16(wds[c] & 0xffffu) << 16) | (0xffffu - uint32_t(q))};
-            dk[q + 1] = Key32{(ord16_from_bf16(wds[c] >> 16) << 16) | (0xffffu - uint32_t(q + 1))};
+        for (int v = 0; v < N / 8; ++v) {
+            const uint4 raw = reinterpret_cast<const uint4 *>(src)[v];
+            pair(raw.x, 8 * v); pair(raw.y, 8 * v + 2); pair(raw.z, 8 * v + 4); pair(raw.w, 8 * v + 6);
         }
+    } else {
+        const uint2 raw = *reinterpret_cast<const uint2 *>(src);
+        pair(raw.x, 0); pair(raw.y, 2);
     }
 }
-
 
 // Decode one row: content indices (before CAPE; a no-op entry reports its rank) and positive
 // weights (zero for an inactive token), in canonical order.
@@ -247,6 +278,7 @@ __device__ __forceinline__ void thread_decode(const T *src, const float rho, int
     // entries of score -inf: a padded candidate sorts with the masked ones and, like them, ends as a no-op entry.
     constexpr int KD = K < P ? K : P;
     constexpr int NB = P / KD;                // digit blocks of KD logits
+    constexpr int V = KD < 8 ? KD : 8;        // logits of one vector load (16-bit types; two loads of four for float)
     constexpr float LOG2E = 1.4426950408889634f;
     constexpr float LN2 = 0.6931471805599453f;
     static_assert(P % KD == 0 && (K & (K - 1)) == 0 && (KD & (KD - 1)) == 0 && K >= 2, "K and min(K, P) powers of two, P a multiple of min(K, P)");
@@ -258,35 +290,31 @@ __device__ __forceinline__ void thread_decode(const T *src, const float rho, int
     int stride = 1;
 
     auto digit = [&](const int u) __attribute__((always_inline)) {
-        // ---- digit u: keys, log-sum-exp, sorted Top-K -------------------------------------------
-        // Passes over the row's P logits (L1-resident after the first); nothing but the keys stays in registers.
-        // Rolled digit loop (three or more digits): keys, then the sum of exponentials; the maximum the sum needs is
-        // the value of the best key (8 % faster at U = 3, P = 32, K = 8).  Unrolled (two digits of 64 logits): a
-        // maximum pass first, the keys last, which keeps the 64 keys out of the way of the exponentials (the
-        // two-pass order is 2.5 % slower there).
-        constexpr bool MAX_FROM_KEYS = U >= 3;
-        DKey dk[P];
-        float xmax = -INFINITY;
-        auto sort_keys = [&]() __attribute__((always_inline)) {
-            rn_make_keys<T, P>(src + u * P, dk);
-            static_for<0, NB>([&](auto BI) __attribute__((always_inline)) { oem_sort_desc<KD>(dk + decltype(BI)::value * KD); });
-            static_for<1, NB>([&](auto BI) __attribute__((always_inline)) { fold_topk<KD>(dk, dk + decltype(BI)::value * KD); });
-        };
-        if constexpr (MAX_FROM_KEYS) {
-            sort_keys();
-            xmax = digit_value<T>(dk[0]);
-        } else {
-            rn_for_each_logit<T, P>(src + u * P, [&](int, float x) { xmax = fmaxf(xmax, x); });
+        // ---- digit u: sorted Top-K, then the log-sum-exp with the best key as its maximum -------------------------
+        // The loops over the row (a block of KD logits, a vector of logits) are unrolled only where the row is short: the
+        // sorting networks are long, and every instance is code to fetch.  The row is in the L1 after the first pass.
+        constexpr int UNROLL = P <= 32 && KD <= 8 ? 32 : 1;
+        DKey dk[KD], blk[KD];
+        const T *row = src + u * P;
+        rn_make_keys<T, KD>(row, 0, dk);
+        oem_sort_desc<KD>(dk);
+#pragma unroll UNROLL
+        for (int q = KD; q < P; q += KD) {
+            rn_make_keys<T, KD>(row + q, q, blk);
+            oem_sort_desc<KD>(blk);
+            fold_topk<KD>(dk, blk);
         }
+        const float xmax = digit_value<T>(dk[0]);
         if (xmax == -INFINITY) {
             inactive = true;
         } else {
             float s = 0.f;
             const float off = xmax * LOG2E;
-            rn_for_each_logit<T, P>(src + u * P, [&](int, float x) { s += fast_ex2(fmaf(x, LOG2E, -off)); });
+#pragma unroll UNROLL
+            for (int q = 0; q < P; q += V)
+                rn_for_each_logit<T, V>(row + q, [&](int, float x) { s += fast_ex2(fmaf(x, LOG2E, -off)); });
             lse_total += xmax + fast_lg2(s) * LN2;
         }
-        if constexpr (!MAX_FROM_KEYS) sort_keys();
         // dk[0..KD) = this digit's KD best logits, sorted descending
 
         if (u == 0) {
@@ -332,16 +360,8 @@ __device__ __forceinline__ void thread_decode(const T *src, const float rho, int
         }
         stride *= P;
     };
-    if constexpr (U >= 3) {
-        // three or more digits: the loop stays rolled.  The straight-line sorting networks are long, and with
-        // the body emitted once instruction fetch stops setting the pace (10 % faster at U = 3, P = 32, K = 8;
-        // at U = 2, P = 64, K = 16 the rolled form needs more registers and is slower)
 #pragma unroll 1
-        for (int u = 0; u < U; ++u) digit(u);
-    } else {
-#pragma unroll
-        for (int u = 0; u < U; ++u) digit(u);
-    }
+    for (int u = 0; u < U; ++u) digit(u);
 
     // ---- weights and stores --------------------------------------------------------------------
     float logq[K];
@@ -383,35 +403,6 @@ __device__ __forceinline__ void fold_topk_xlane(Key *a, int m) {
     bitonic_merge_desc<K>(a);
 }
 
-template <typename T, int K>
-__device__ __forceinline__ void quad_make_keys(const T *src, int p0, Key64 *dk) {
-    rn_for_each_logit<T, K>(src, [&](int q, float x) { dk[q] = Key64{rn_ord(x + 0.0f), ~uint32_t(p0 + q)}; });
-}
-template <typename T, int K>
-__device__ __forceinline__ void quad_make_keys(const T *src, int p0, Key32 *dk) {
-    if constexpr (K >= 8) {
-#pragma unroll
-        for (int v = 0; v < K / 8; ++v) {
-            const uint4 raw = reinterpret_cast<const uint4 *>(src)[v];
-            const uint32_t wds[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int q = 8 * v + 2 * c;
-                dk[q] = Key32{(ord16_from_bf16(wds[c] & 0xffffu) << 16) | (0xffffu - uint32_t(p0 + q))};
-                dk[q + 1] = Key32{(ord16_from_bf16(wds[c] >> 16) << 16) | (0xffffu - uint32_t(p0 + q + 1))};
-            }
-        }
-    } else {
-        const uint2 raw = *reinterpret_cast<const uint2 *>(src);  // K == 4 sixteen-bit logits
-        const uint32_t wds[2] = {raw.x, raw.y};
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            dk[2 * c] = Key32{(ord16_from_bf16(wds[c] & 0xffffu) << 16) | (0xffffu - uint32_t(p0 + 2 * c))};
-            dk[2 * c + 1] = Key32{(ord16_from_bf16(wds[c] >> 16) << 16) | (0xffffu - uint32_t(p0 + 2 * c + 1))};
-        }
-    }
-}
-
 template <typename T, int U, int P, int K>
 __device__ __forceinline__ void quad_decode(const T *src, const float rho, const int gl, int (&content)[K],
                                             float (&weight)[K]) {
@@ -435,7 +426,7 @@ __device__ __forceinline__ void quad_decode(const T *src, const float rho, const
     for (int u = 0; u < U; ++u) {
         const T *mine = src + u * P + gl * K;  // this lane's K logits of digit u
         DKey dk[K];
-        quad_make_keys<T, K>(mine, gl * K, dk);
+        rn_make_keys<T, K>(mine, gl * K, dk);
         oem_sort_desc<K>(dk);
 #pragma unroll 1
         for (int m = 1; m <= 2; m <<= 1) fold_topk_xlane<K>(dk, m);
@@ -446,12 +437,7 @@ __device__ __forceinline__ void quad_decode(const T *src, const float rho, const
         } else {
             float s = 0.f;
             const float off = xmax * LOG2E;
-            if constexpr (Raw<T>::wide || K >= 8) {
-                rn_for_each_logit<T, K>(mine, [&](int, float x) { s += fast_ex2(fmaf(x, LOG2E, -off)); });
-            } else {
-#pragma unroll
-                for (int q = 0; q < K; ++q) s += fast_ex2(fmaf(rn_to_float<T>(mine[q]), LOG2E, -off));
-            }
+            rn_for_each_logit<T, K>(mine, [&](int, float x) { s += fast_ex2(fmaf(x, LOG2E, -off)); });
             s += __shfl_xor_sync(RN_FULL, s, 1);
             s += __shfl_xor_sync(RN_FULL, s, 2);
             lse_total += xmax + fast_lg2(s) * LN2;

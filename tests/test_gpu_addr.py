@@ -181,3 +181,16 @@ def test_specialised_and_general_kernels_agree(U, P, K, dtype):
         ref_idx, ref_val = orc.topk_addr(logits.float().permute(0, 2, 3, 4, 1), E, pos, K, renorm)
         assert torch.equal(a[0][:, :, :K].cpu(), ref_idx)
         assert_close_stats("val", a[1][:, :, :K].cpu(), ref_val, atol=1e-6, rtol=2e-5, max_err_rate=0.0)
+
+
+NEW_INSTANCES = [(2, 64, 8), (2, 64, 32), (2, 32, 8), (3, 8, 8)]
+
+
+@pytest.mark.parametrize("U,P,K", NEW_INSTANCES)
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_further_thread_per_row_instances(U, P, K, dtype):
+    """Instances for more addresses per digit block, fewer and more than one: forward against the general kernel (exact
+    ties included), gradients against the oracle."""
+    test_specialised_and_general_kernels_agree(U, P, K, dtype)
+    if dtype == torch.float32:
+        test_backward_matches_oracle_autograd((1, 2, U, P, 11, K, 1, dtype, 1.0), 0.5, True)
