@@ -128,17 +128,8 @@ __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnList
         const int f = lg == 0 ? 0 : lg == 1 ? rn_fold<1>(r) : lg == 2 ? rn_fold<2>(r) : rn_fold<3>(r);
         return (r << lg) | (own ^ f);
     };
-    {
-        const int ul = tid % LPU, ch = grp * CS + ul * 4;
-        const float *src = p.slot_in ? p.slot_in + int64_t(bh) * p.A * C + ch : nullptr;
-#pragma unroll 1
-        for (int r = tid / LPU; r < rows; r += RN_AP_THREADS / LPU) {
-            const int a = slot_of(r);
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (src != nullptr && ch < C && a < p.A) v = *reinterpret_cast<const float4 *>(src + int64_t(a) * C);
-            *reinterpret_cast<float4 *>(S + size_t(r) * ROW + ul * 16) = v;
-        }
-    }
+    const int words = rn_touch_words(p.lr);
+    const uint32_t *touch = p.touch ? p.touch + ((int64_t(bh) << lg) + own) * 2 * words : nullptr;
     __syncthreads();
     if (N > 1) rn_cluster_sync();  // every CTA's barriers are set up before the first remote arrival
 
@@ -251,6 +242,26 @@ __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnList
         const int ch0 = grp * CS + int(lane_off) / 4, ch1 = grp * CS + int(lane_off ^ HALF) / 4;
         T *y = static_cast<T *>(p.y) + b * p.yb + h * p.yh;
         const int lq = 31 - __clz(Lq);
+        {   // the rows into shared memory, eight requests of a thread at a time; the service warps fetch the first step meanwhile
+            constexpr int LD = CS / 4, STEP = RN_AP_COMPUTE / LD;
+            const int sub = tid % LD, ch = grp * CS + sub * 4;
+            const float *src = p.slot_in && ch < C ? p.slot_in + int64_t(bh) * p.A * C + ch : nullptr;
+#pragma unroll 1
+            for (int r0 = tid / LD; r0 < rows; r0 += 8 * STEP) {
+                float4 v[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int r = r0 + i * STEP, a = slot_of(r);
+                    const bool on = r < rows && src != nullptr && a < p.A && (touch == nullptr || (touch[r >> 5] >> (r & 31) & 1u) != 0);
+                    v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (on) v[i] = *reinterpret_cast<const float4 *>(src + int64_t(a) * C);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (r0 + i * STEP < rows) *reinterpret_cast<float4 *>(S + size_t(r0 + i * STEP) * ROW + sub * 16) = v[i];
+            }
+            if (rn_compute_sync(false)) failed = true;
+        }
         int blk = -1;
 #pragma unroll 1
         for (int step = 0;; ++step) {
@@ -387,7 +398,8 @@ __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnList
 #pragma unroll 1
         for (int r = tid / LPU; r < rows; r += RN_AP_THREADS / LPU) {
             const int a = slot_of(r);
-            if (ch < C && a < p.A) *reinterpret_cast<float4 *>(dst + int64_t(a) * C) = *reinterpret_cast<const float4 *>(S + size_t(r) * ROW + ul * 16);
+            const bool on = touch == nullptr || (touch[words + (r >> 5)] >> (r & 31) & 1u) != 0;
+            if (on && ch < C && a < p.A) *reinterpret_cast<float4 *>(dst + int64_t(a) * C) = *reinterpret_cast<const float4 *>(S + size_t(r) * ROW + ul * 16);
         }
     }
     if (N > 1) rn_cluster_sync();  // nobody's shared memory goes away while a store or arrival to it may be under way

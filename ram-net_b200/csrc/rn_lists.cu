@@ -377,6 +377,7 @@ __global__ void __launch_bounds__(RN_GAINS_THREADS) rn_gains_kernel(const RnList
     constexpr int NT = RN_GAINS_THREADS, N = 1 << LG;
     extern __shared__ __align__(128) unsigned char dyn[];
     __shared__ __align__(8) uint64_t mbar[2];
+    __shared__ uint32_t touched[2][RN_LST_ROWS / 32];
     const int own = blockIdx.x & (N - 1), bh = blockIdx.x >> LG, tid = threadIdx.x;
     const int A = p.A, rows = 1 << p.lr;
 
@@ -404,6 +405,11 @@ __global__ void __launch_bounds__(RN_GAINS_THREADS) rn_gains_kernel(const RnList
     int nblk = rn_steps_of(cur) > 1 ? 0 : 1, nst = rn_steps_of(cur) > 1 ? 1 : 0;
     uint4 nxt = rn_step_entry(p, first, recs, nblk, nst, own);
     const float *mass_in = p.mass_in ? p.mass_in + int64_t(bh) * A : nullptr;
+    if (p.touch != nullptr)
+        for (int i = tid; i < 2 * RN_LST_ROWS / 32; i += NT) touched[0][i] = 0;  // both rows of the array
+    auto touch = [&](int set, uint32_t r) {
+        if (!(touched[set][r >> 5] & (1u << (r & 31)))) atomicOr(&touched[set][r >> 5], 1u << (r & 31));
+    };
 #pragma unroll 1
     for (int r = tid; r < rows; r += NT) {
         const int a = rn_slot_of<LG>(own, r);
@@ -423,7 +429,7 @@ __global__ void __launch_bounds__(RN_GAINS_THREADS) rn_gains_kernel(const RnList
         unsigned char *lst = buf + size_t(step & 1) * p.whole_max;
         unsigned char *glst = recs + blk * p.blk_bytes + data_at + (size_t(cur.x & 0xffffu) << 4);
         RnListHdr hd = *reinterpret_cast<const RnListHdr *>(lst);
-        if (failed) hd.len = hd.nS = hd.nM = hd.nR = hd.nF = 0;  // stays in step with the cluster and does nothing else
+        if (failed) hd.len = hd.nS = hd.nM = hd.nW = hd.nR = hd.nF = 0;  // stays in step with the cluster and does nothing else
         uint2 *W = reinterpret_cast<uint2 *>(lst + (uint32_t(hd.atW) << 4)), *R = reinterpret_cast<uint2 *>(lst + (uint32_t(hd.atR) << 4));
         uint2 *gW = reinterpret_cast<uint2 *>(glst + (uint32_t(hd.atW) << 4)), *gR = reinterpret_cast<uint2 *>(glst + (uint32_t(hd.atR) << 4));
         float2 *aw = reinterpret_cast<float2 *>(R + ((hd.nR + 1) & ~1));
@@ -431,6 +437,12 @@ __global__ void __launch_bounds__(RN_GAINS_THREADS) rn_gains_kernel(const RnList
         const uint16_t *tok = reinterpret_cast<const uint16_t *>(lst + 16), *start = tok + len + 1;
         const uint16_t *fix = reinterpret_cast<const uint16_t *>(aw + ((hd.nW + 1) & ~1));
 
+        if (p.touch != nullptr) {
+#pragma unroll 1
+            for (int i = tid; i < hd.nR; i += NT) touch(0, (R[i].y >> 31) != 0 ? R[i].y & 0x7ffu : R[i].y >> p.rs);
+#pragma unroll 1
+            for (int q = tid; q < hd.nW; q += NT) touch(1, W[q].y & 0x7ffu);
+        }
         if (MA) {  // weight times mass for the reads that no write of the step precedes
 #pragma unroll 1
             for (int i = tid; i < hd.nR; i += NT) {
@@ -542,6 +554,14 @@ __global__ void __launch_bounds__(RN_GAINS_THREADS) rn_gains_kernel(const RnList
         const int a = rn_slot_of<LG>(own, r);
         if (a < A) mass_out[a] = mass[r];
     }
+    if (p.touch != nullptr) {  // the loop ended with a barrier
+        const int words = rn_touch_words(p.lr);
+        for (int i = tid; i < words; i += NT) {
+            uint32_t *out = p.touch + blockIdx.x * 2 * words + i;
+            out[0] = touched[0][i] | touched[1][i];
+            out[words] = touched[1][i];
+        }
+    }
     if (MA && N > 1) rn_cluster_sync();  // the sums may still be read from another CTA
 }
 
@@ -593,7 +613,8 @@ bool rn_list_plan(int64_t B, int64_t H, int64_t T, int64_t A, int64_t C, int64_t
         for (int lg = 0; (1 << lg) <= RN_LST_OWNERS && !found; ++lg) found = fits(lg, L);
     if (!found) return false;
     pl->off_first = size_t(B * H) * pl->nblocks * pl->blk_bytes;
-    pl->total = rn_align(pl->off_first + (size_t(B * H) * pl->nblocks << pl->lg) * 16, 256);
+    pl->off_touch = pl->off_first + (size_t(B * H) * pl->nblocks << pl->lg) * 16;
+    pl->total = rn_align(pl->off_touch + (size_t(B * H) << pl->lg) * 8 * rn_touch_words(pl->lr), 256);
     return true;
 }
 

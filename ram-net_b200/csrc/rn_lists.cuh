@@ -92,7 +92,7 @@ struct RnListPlan {
     uint32_t whole_max;           // likewise, the whole list
     uint32_t step_max;            // largest step (all owners)
     size_t smem_lists, smem_gains, smem_apply;
-    size_t off_first, total;      // workspace: first-step table, bytes
+    size_t off_first, off_touch, total;  // workspace: first-step table, touched rows, bytes
 };
 __host__ __device__ __forceinline__ uint32_t rn_list_data_at(int L, int lg) { return (uint32_t(L) << lg) * 16u; }
 
@@ -124,6 +124,9 @@ struct RnListParams {
     int *status;
     unsigned char *recs;
     uint4 *first;
+    // optional, for a short sequence on a state that is updated in place: [bh][owner][2][rn_touch_words] bits of the rows that
+    // the call reads or writes and of those that it writes; the others stay in global memory
+    uint32_t *touch;
 };
 
 // walks the steps of a (b,h): the entry of an owner in step st of block blk; all zero behind the last block
@@ -146,6 +149,8 @@ __device__ __forceinline__ uint32_t rn_mapa(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void rn_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+
+__host__ __device__ __forceinline__ int rn_touch_words(int lr) { return lr < 5 ? 1 : 1 << (lr - 5); }
 
 // false: not a shape of these kernels
 bool rn_list_plan(int64_t B, int64_t H, int64_t T, int64_t A, int64_t C, int64_t Kw, int64_t Kr, int mass_aware, RnListPlan *pl);

@@ -74,3 +74,20 @@ def test_event_lists_match_a_sequential_reference(A, T, C, K, pool, dtype, maske
     assert float((m.cpu().double() - rm).abs().max()) <= 8 * tol * float(rm.abs().max())
     out = {torch.float32: 64 * tol, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -10}[dtype]
     assert float((y.cpu().double() - ry).norm() / ry.norm()) <= out
+
+
+@pytest.mark.parametrize("T", [1, 40, 129])
+def test_in_place_moves_touched_rows_only_and_leaves_the_others(T):
+    """Few events on a large state updated in place: the same results as the copying form, untouched rows bit for bit."""
+    ops()
+    B, H, A, C, K = 2, 3, 4096, 64, 6
+    g = torch.Generator().manual_seed(T)
+    idx = torch.randint(A, (B, T, H, 2 * K), generator=g).to(torch.int32).permute(0, 2, 3, 1).cuda()
+    val = (torch.rand(B, T, H, 2 * K, generator=g) * 0.4 + 0.01).permute(0, 2, 3, 1).cuda()
+    x, gamma = torch.randn(B, H, T, C, generator=g).cuda(), torch.randn(B, H, T, generator=g).cuda()
+    slot, mass = torch.randn(B, H, A, C, generator=g).cuda(), (torch.rand(B, H, A, generator=g) + 0.1).cuda()
+    for ma in (False, True):
+        want = torch.ops.ramnet_ops.gsu_forward(idx, val, x, gamma, slot, mass, None, K, K, ma, 1e-6)
+        s, m = slot.clone(), mass.clone()
+        y = torch.ops.ramnet_ops.gsu_forward_(idx, val, x, gamma, s, m, None, K, K, ma, 1e-6)
+        assert torch.equal(y, want[0]) and torch.equal(s, want[1]) and torch.equal(m, want[2])
