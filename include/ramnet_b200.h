@@ -178,6 +178,16 @@ int rn_decode_step_pos(const void *w_addr, const void *r_addr, const void *x, co
                        int64_t B, int64_t H, int64_t U, int64_t P, int64_t C, int64_t E,
                        int64_t Kw, int64_t Kr, double w_re_norm, double r_re_norm,
                        int mass_aware, double eps, int device, void *stream);
+/* `steps` consecutive steps on one state in one launch, as that many calls with the positions advanced by one in between:
+ *  step_strides : (steps > 1) 5 element strides between the steps' w_addr, r_addr, x, gamma and gate_logits
+ *  y            : (steps, B, H, C) contiguous; pos itself is not changed; w_scale / r_scale: for a single step. */
+int rn_decode_steps(const void *w_addr, const void *r_addr, const void *x, const void *gamma, int dtype,
+                    float *slot, float *mass, const uint8_t *mask, const void *pos, int pos_kind, int64_t pos_stride,
+                    void *y, const float *norm_weight, const void *gate_logits, double norm_eps,
+                    const void *w_scale, const void *r_scale, const int64_t *batch_strides, int64_t steps,
+                    const int64_t *step_strides, int64_t B, int64_t H, int64_t U, int64_t P, int64_t C, int64_t E,
+                    int64_t Kw, int64_t Kr, double w_re_norm, double r_re_norm, int mass_aware, double eps, int device,
+                    void *stream);
 
 /*
  * Prefill (T > 1) gated sparse update + read over decoded addresses.

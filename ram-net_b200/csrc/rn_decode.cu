@@ -8,9 +8,12 @@
 //       read rows by per-lane loads in flight at the same time; a CTA's warps draw pairs from a shared counter.
 //   rn_decode_fast_kernel  (U,P,K) = (2,64,16), (3,32,8), (2,16,4) with 32-bit or 16-bit logits: one CTA per
 //       16 pairs, four lanes per address on warps 0-3, then warp w owns pairs 2w and 2w+1; rows as above.
-//   rn_decode_kernel       any U <= 8, P <= 128, K <= 128, C <= 1024: one CTA per pair, warp 0 / 1 decode the
-//       write / read address, rows updated in place (128-bit accesses when C is a multiple of 4), reads
-//       gathered after a CTA barrier and reduced over K in a fixed order.
+//   rn_decode_kernel       any U <= 8, P <= 128, K <= 128, C <= 1024: one CTA per pair, two warps decode the
+//       write / read address, four update the rows in place (128-bit accesses when C is a multiple of 4), gather the
+//       reads after a barrier and reduce them over K in a fixed order.
+//
+// All three take several consecutive steps in one launch (rn_decode_steps): a (batch, head) pair depends on no other one,
+// so whoever owns a pair goes through its steps without a grid-wide barrier.
 //
 // A read of a slot written in the same step sees the new value.  State offsets are 64-bit: B*H*A*C may
 // exceed 2^31 elements.  A bounded wait that runs out is reported through the device's status word; slot
@@ -20,7 +23,7 @@
 #include "rn_prefill.cuh"
 #include "rn_gsu.cuh"
 
-constexpr int RN_DEC_WARPS = 4;
+constexpr int RN_DEC_WARPS = 4, RN_DEC_THREADS = (RN_DEC_WARPS + 2) * 32;  // row warps; these and two decoders
 constexpr int RN_DEC_CMAX = 1024;
 
 struct RnDecodeParams {
@@ -37,6 +40,9 @@ struct RnDecodeParams {
     int64_t ld_addr[2], ld_x, ld_gamma, ld_gate;
     float norm_eps;
     int B, H, U, P, C, E, A;
+    // consecutive steps of one launch and the element strides between their inputs and outputs
+    int steps;
+    int64_t st_addr[2], st_x, st_gamma, st_gate, st_y;
     int K[2];
     float re_norm[2];
     int mass_aware;
@@ -51,14 +57,16 @@ __device__ __forceinline__ int64_t rn_in_row(const RnDecodeParams &p, const int 
     return b * ld + int64_t(h) * per_head;
 }
 
+// Four warps move the rows, two more decode the write and the read address; with several steps the decoders are one step
+// ahead.  A warp requests four rows before it uses the first; gains and read coefficients are computed one per lane.
 template <typename T, int KPL, int PPL>
-__global__ void __launch_bounds__(RN_DEC_WARPS * 32) rn_decode_kernel(const RnDecodeParams p) {
-    extern __shared__ float dyn[];  // xs[C] | yred[4][C]
+__global__ void __launch_bounds__(RN_DEC_THREADS) rn_decode_kernel(const RnDecodeParams p) {
+    extern __shared__ float dyn[];  // xs[2][C] | yred[4][C]
     __shared__ RnPairTable tabs[2];
     __shared__ RnWarpScratch scratch[2];
     __shared__ int row_off[RN_KMAX + 1];
-    __shared__ int sel_slot[2][RN_KMAX];
-    __shared__ float sel_val[2][RN_KMAX];
+    __shared__ int sel_slot[2][2][RN_KMAX];  // by parity of the step
+    __shared__ float sel_val[2][2][RN_KMAX];
     __shared__ float red[RN_DEC_WARPS][2];
     __shared__ float bcast;
 
@@ -66,152 +74,229 @@ __global__ void __launch_bounds__(RN_DEC_WARPS * 32) rn_decode_kernel(const RnDe
     const int b = bh / p.H, h = bh % p.H;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int C = p.C;
-    T *y = static_cast<T *>(p.y) + int64_t(bh) * C;
 
     if (p.mask != nullptr && p.mask[b] == 0) {
-        for (int c = tid; c < C; c += blockDim.x) y[c] = rn_from_float<T>(0.f);
+        for (int step = 0; step < p.steps; ++step) {
+            T *y = static_cast<T *>(p.y) + step * p.st_y + int64_t(bh) * C;
+            for (int c = tid; c < C; c += RN_DEC_THREADS) y[c] = rn_from_float<T>(0.f);
+        }
         return;
     }
 
-    float *xs = dyn;
-    float *yred = dyn + C;
+    float *yred = dyn + 2 * C;
 
     rn_build_pairs(&tabs[0], p.K[0], row_off);
     if (p.K[1] != p.K[0]) rn_build_pairs(&tabs[1], p.K[1], row_off);
-    const RnPairTable *tab_r = (p.K[1] != p.K[0]) ? &tabs[1] : &tabs[0];
 
-    if (warp < 2) {
-        RnDigitLoader<T> load;
-        load.base = static_cast<const T *>(warp == 0 ? p.w_addr : p.r_addr) + rn_in_row(p, bh, p.ld_addr[warp == 0 ? 0 : 1], p.U * p.P);
-        load.su = p.P;
-        load.sp = 1;
-        const int K = p.K[warp];
-        const RnDecoded<KPL> d =
-            rn_warp_decode<KPL, PPL>(load, p.U, p.P, K, p.re_norm[warp], &scratch[warp], warp == 0 ? &tabs[0] : tab_r, lane);
-        const int shift = (h < p.E) ? rn_pos_mod(rn_pos_at(p.pos, b, 0), p.A) : 0;
+    if (warp >= RN_DEC_WARPS) {
+        // ================================ decoders ==========================================================
+        const int which = warp - RN_DEC_WARPS, K = p.K[which];
+        const RnPairTable *tab = &tabs[p.K[1] != p.K[0] ? which : 0];
+        const int pos = h < p.E ? rn_pos_at(p.pos, b, 0) : 0;
+        const T *src = static_cast<const T *>(which ? p.r_addr : p.w_addr) + rn_in_row(p, bh, p.ld_addr[which], p.U * p.P);
+#pragma unroll 1
+        for (int step = 0; step < p.steps; ++step) {
+            RnDigitLoader<T> load;
+            load.base = src + step * p.st_addr[which];
+            load.su = p.P;
+            load.sp = 1;
+            const RnDecoded<KPL> d = rn_warp_decode<KPL, PPL>(load, p.U, p.P, K, p.re_norm[which], &scratch[which], tab, lane);
+            const int shift = (h < p.E) ? rn_pos_mod(pos + step, p.A) : 0;
 #pragma unroll
-        for (int r = 0; r < KPL; ++r) {
-            const int e = lane * KPL + r;
-            if (e < K) {
-                sel_slot[warp][e] = rn_cape(d.idx[r], shift, p.A);
-                sel_val[warp][e] = d.val[r];
+            for (int r = 0; r < KPL; ++r) {
+                const int e = lane * KPL + r;
+                if (e < K) {
+                    sel_slot[step & 1][which][e] = rn_cape(d.idx[r], shift, p.A);
+                    sel_val[step & 1][which][e] = d.val[r];
+                }
             }
+            __syncthreads();  // the step's addresses are there, those of the step before have been used
         }
-    } else {
-        const T *x = static_cast<const T *>(p.x) + rn_in_row(p, bh, p.ld_x, C);
-        for (int c = tid - 64; c < C; c += 64) xs[c] = rn_to_float<T>(x[c]);
+        return;
     }
-    for (int c = tid; c < RN_DEC_WARPS * C; c += blockDim.x) yred[c] = 0.f;
-    __syncthreads();
 
-    const float gamma = rn_to_float<T>(static_cast<const T *>(p.gamma)[rn_in_row(p, bh, p.ld_gamma, 1)]);
+    // ================================ rows ==================================================================
+    // the decoders have left once the last step's addresses are there: what follows are barriers of these four warps
+    auto rows_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(RN_DEC_WARPS * 32) : "memory"); };
     float *slot = p.slot + int64_t(bh) * p.A * C;
     float *mass = p.mass + int64_t(bh) * p.A;
-    const bool vec4 = (C & 3) == 0;
+    const bool vec4 = (C & 3) == 0, epilogue = p.norm_weight != nullptr || p.gate != nullptr;
+#pragma unroll 1
+    for (int step = 0; step < p.steps; ++step) {
+        float *xs = dyn + (step & 1) * C;
+        T *y = static_cast<T *>(p.y) + step * p.st_y + int64_t(bh) * C;
+        {
+            const T *x = static_cast<const T *>(p.x) + step * p.st_x + rn_in_row(p, bh, p.ld_x, C);
+            for (int c = tid; c < C; c += RN_DEC_WARPS * 32) xs[c] = rn_to_float<T>(x[c]);
+        }
+        const float gamma = rn_to_float<T>(static_cast<const T *>(p.gamma)[step * p.st_gamma + rn_in_row(p, bh, p.ld_gamma, 1)]);
+        __syncthreads();
+        const int *ws = sel_slot[step & 1][0], *rs = sel_slot[step & 1][1];
+        const float *wv = sel_val[step & 1][0], *rv = sel_val[step & 1][1];
 
-    // ---- write: gated update of the selected rows ---------------------------------------------
-    for (int k = warp; k < p.K[0]; k += RN_DEC_WARPS) {
-        const float w = sel_val[0][k];
-        if (w == 0.f) continue;
-        const int a = sel_slot[0][k];
-        const RnGate g = rn_gate(w, gamma, mass[a], p.eps);
-        float *row = slot + int64_t(a) * C;
+        // ---- write: gated update of the selected rows; lane i of a group of four rows has the gain of row i ---------
         if (vec4) {
-            for (int c = lane * 4; c < C; c += 128) {
-                float4 s = *reinterpret_cast<float4 *>(row + c);
-                const float4 xv = *reinterpret_cast<const float4 *>(xs + c);
-                s.x = fmaf(g.gain, xv.x - s.x, s.x);
-                s.y = fmaf(g.gain, xv.y - s.y, s.y);
-                s.z = fmaf(g.gain, xv.z - s.z, s.z);
-                s.w = fmaf(g.gain, xv.w - s.w, s.w);
-                *reinterpret_cast<float4 *>(row + c) = s;
+#pragma unroll 1
+            for (int k0 = warp; k0 < p.K[0]; k0 += 4 * RN_DEC_WARPS) {
+                const int kl = k0 + (lane & 3) * RN_DEC_WARPS;
+                const float w = kl < p.K[0] ? wv[kl] : 0.f;
+                const int a = kl < p.K[0] ? ws[kl] : 0;
+                const float m = w != 0.f ? mass[a] : 0.f;
+                float gain = 0.f, after = 0.f;
+#pragma unroll 1
+                for (int c = lane * 4; c < C + lane * 4; c += 128) {  // C / 128 rounds, rounded up, in every lane
+                    float4 s[4];
+                    float *row[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int ai = __shfl_sync(RN_FULL, a, i);
+                        const bool on = __shfl_sync(RN_FULL, w, i) != 0.f && c < C;
+                        row[i] = on ? slot + int64_t(ai) * C + c : nullptr;
+                        if (on) s[i] = *reinterpret_cast<const float4 *>(row[i]);
+                    }
+                    if (c == lane * 4 && w != 0.f) {
+                        const RnGate g = rn_gate(w, gamma, m, p.eps);
+                        gain = g.gain;
+                        after = g.mass;
+                    }
+                    const float4 xv = c < C ? *reinterpret_cast<const float4 *>(xs + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float g = __shfl_sync(RN_FULL, gain, i);
+                        if (row[i] == nullptr) continue;
+                        s[i].x = fmaf(g, xv.x - s[i].x, s[i].x);
+                        s[i].y = fmaf(g, xv.y - s[i].y, s[i].y);
+                        s[i].z = fmaf(g, xv.z - s[i].z, s[i].z);
+                        s[i].w = fmaf(g, xv.w - s[i].w, s[i].w);
+                        *reinterpret_cast<float4 *>(row[i]) = s[i];
+                    }
+                }
+                if (lane < 4 && w != 0.f) mass[a] = after;
             }
         } else {
-            for (int c = lane; c < C; c += 32) row[c] = fmaf(g.gain, xs[c] - row[c], row[c]);
+            for (int k = warp; k < p.K[0]; k += RN_DEC_WARPS) {
+                const float w = wv[k];
+                if (w == 0.f) continue;
+                const int a = ws[k];
+                const RnGate g = rn_gate(w, gamma, mass[a], p.eps);
+                float *row = slot + int64_t(a) * C;
+                for (int c = lane; c < C; c += 32) row[c] = fmaf(g.gain, xs[c] - row[c], row[c]);
+                __syncwarp();
+                if (lane == 0) mass[a] = g.mass;
+            }
         }
-        __syncwarp();
-        if (lane == 0) mass[a] = g.mass;
-    }
-    __syncthreads();
+        rows_sync();
 
-    // ---- read: weighted sum of the selected rows (after this step's writes) --------------------
-    float sum_r = 0.f, sum_rm = 0.f;
-    float *acc = yred + warp * C;
-    for (int k = warp; k < p.K[1]; k += RN_DEC_WARPS) {
-        const float r = sel_val[1][k];
-        if (r == 0.f) continue;
-        const int a = sel_slot[1][k];
-        float coef = r;
+        // ---- read: weighted sum of the selected rows (after this step's writes) --------------------
+        float sum_r = 0.f, sum_rm = 0.f;
+        float *acc = yred + warp * C;
+        if (vec4) {
+#pragma unroll 1
+            for (int c = lane * 4; c < C + lane * 4; c += 128) {
+                float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+                for (int k0 = warp; k0 < p.K[1]; k0 += 4 * RN_DEC_WARPS) {
+                    const int kl = k0 + (lane & 3) * RN_DEC_WARPS;
+                    const float r = kl < p.K[1] ? rv[kl] : 0.f;
+                    const int a = kl < p.K[1] ? rs[kl] : 0;
+                    float4 s[4];
+                    bool on[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int ai = __shfl_sync(RN_FULL, a, i);
+                        on[i] = __shfl_sync(RN_FULL, r, i) != 0.f && c < C;
+                        if (on[i]) s[i] = *reinterpret_cast<const float4 *>(slot + int64_t(ai) * C + c);
+                    }
+                    float coef = r;
+                    if (p.mass_aware) {
+                        coef = r != 0.f ? r * mass[a] : 0.f;
+                        if (c == lane * 4) {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                sum_r += __shfl_sync(RN_FULL, r, i);
+                                sum_rm += __shfl_sync(RN_FULL, coef, i);
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float f = __shfl_sync(RN_FULL, coef, i);
+                        if (!on[i]) continue;
+                        o.x = fmaf(f, s[i].x, o.x);
+                        o.y = fmaf(f, s[i].y, o.y);
+                        o.z = fmaf(f, s[i].z, o.z);
+                        o.w = fmaf(f, s[i].w, o.w);
+                    }
+                }
+                if (c < C) *reinterpret_cast<float4 *>(acc + c) = o;
+            }
+        } else {
+            for (int c = lane; c < C; c += 32) acc[c] = 0.f;
+            for (int k = warp; k < p.K[1]; k += RN_DEC_WARPS) {
+                const float r = rv[k];
+                if (r == 0.f) continue;
+                const int a = rs[k];
+                float coef = r;
+                if (p.mass_aware) {
+                    coef = r * mass[a];
+                    sum_r += r;
+                    sum_rm += coef;
+                }
+                const float *row = slot + int64_t(a) * C;
+                for (int c = lane; c < C; c += 32) acc[c] = fmaf(coef, row[c], acc[c]);
+            }
+        }
+        if (lane == 0) {
+            red[warp][0] = sum_r;
+            red[warp][1] = sum_rm;
+        }
+        rows_sync();
+
+        float scale = 1.f;
         if (p.mass_aware) {
-            coef = r * mass[a];
-            sum_r += r;
-            sum_rm += coef;
-        }
-        const float *row = slot + int64_t(a) * C;
-        if (vec4) {
-            for (int c = lane * 4; c < C; c += 128) {
-                const float4 s = *reinterpret_cast<const float4 *>(row + c);
-                float4 o = *reinterpret_cast<float4 *>(acc + c);
-                o.x = fmaf(coef, s.x, o.x);
-                o.y = fmaf(coef, s.y, o.y);
-                o.z = fmaf(coef, s.z, o.z);
-                o.w = fmaf(coef, s.w, o.w);
-                *reinterpret_cast<float4 *>(acc + c) = o;
+            float sr = 0.f, srm = 0.f;
+            for (int w = 0; w < RN_DEC_WARPS; ++w) {
+                sr += red[w][0];
+                srm += red[w][1];
             }
-        } else {
-            for (int c = lane; c < C; c += 32) acc[c] = fmaf(coef, row[c], acc[c]);
+            scale = sr / (srm + p.eps);
         }
-    }
-    if (lane == 0) {
-        red[warp][0] = sum_r;
-        red[warp][1] = sum_rm;
-    }
-    __syncthreads();
-
-    float scale = 1.f;
-    if (p.mass_aware) {
-        float sr = 0.f, srm = 0.f;
-        for (int w = 0; w < RN_DEC_WARPS; ++w) {
-            sr += red[w][0];
-            srm += red[w][1];
+        float sq = 0.f;
+        for (int c = tid; c < C; c += RN_DEC_WARPS * 32) {
+            float v = 0.f;
+            for (int w = 0; w < RN_DEC_WARPS; ++w) v += yred[w * C + c];
+            v *= scale;
+            if (epilogue) {
+                yred[c] = v;  // column c is owned by this thread in every pass
+                sq += v * v;
+            } else {
+                y[c] = rn_from_float<T>(v);
+            }
         }
-        scale = sr / (srm + p.eps);
-    }
-    const bool epilogue = p.norm_weight != nullptr || p.gate != nullptr;
-    float sq = 0.f;
-    for (int c = tid; c < C; c += blockDim.x) {
-        float v = 0.f;
-        for (int w = 0; w < RN_DEC_WARPS; ++w) v += yred[w * C + c];
-        v *= scale;
         if (epilogue) {
-            yred[c] = v;  // column c is owned by this thread in every pass
-            sq += v * v;
-        } else {
-            y[c] = rn_from_float<T>(v);
+            float inv_rms = 1.f;
+            if (p.norm_weight != nullptr) {
+                sq = rn_warp_sum(sq);
+                rows_sync();  // red[] is reused
+                if (lane == 0) red[warp][0] = sq;
+                rows_sync();
+                if (tid == 0) {
+                    float s = 0.f;
+                    for (int w = 0; w < RN_DEC_WARPS; ++w) s += red[w][0];
+                    bcast = rsqrtf(s / float(C) + p.norm_eps);
+                }
+                rows_sync();
+                inv_rms = bcast;
+            }
+            const T *gate = p.gate ? static_cast<const T *>(p.gate) + step * p.st_gate + rn_in_row(p, bh, p.ld_gate, C) : nullptr;
+            for (int c = tid; c < C; c += RN_DEC_WARPS * 32) {
+                float v = yred[c];
+                if (p.norm_weight != nullptr) v = v * inv_rms * p.norm_weight[c];
+                if (gate != nullptr) v = v / (1.f + expf(-rn_to_float<T>(gate[c])));
+                y[c] = rn_from_float<T>(v);
+            }
         }
-    }
-    if (!epilogue) return;
-
-    float inv_rms = 1.f;
-    if (p.norm_weight != nullptr) {
-        sq = rn_warp_sum(sq);
-        __syncthreads();  // red[] is reused
-        if (lane == 0) red[warp][0] = sq;
-        __syncthreads();
-        if (tid == 0) {
-            float s = 0.f;
-            for (int w = 0; w < RN_DEC_WARPS; ++w) s += red[w][0];
-            bcast = rsqrtf(s / float(C) + p.norm_eps);
-        }
-        __syncthreads();
-        inv_rms = bcast;
-    }
-    const T *gate = p.gate ? static_cast<const T *>(p.gate) + rn_in_row(p, bh, p.ld_gate, C) : nullptr;
-    for (int c = tid; c < C; c += blockDim.x) {
-        float v = yred[c];
-        if (p.norm_weight != nullptr) v = v * inv_rms * p.norm_weight[c];
-        if (gate != nullptr) v = v / (1.f + expf(-rn_to_float<T>(gate[c])));
-        y[c] = rn_from_float<T>(v);
+        // the barrier at the head of the next step keeps what this one still reads (yred, red) from being written to
     }
 }
 
@@ -230,7 +315,8 @@ __global__ void __launch_bounds__(RN_DEC_WARPS * 32) rn_decode_kernel(const RnDe
 constexpr int RN_DECF_PAIRS = 16;
 constexpr int RN_DECF_THREADS = 256;
 
-template <typename T, int U, int P, int K, int NV>
+// STEPS: several steps per launch
+template <typename T, int U, int P, int K, int NV, bool STEPS>
 __global__ void __launch_bounds__(RN_DECF_THREADS, 2) rn_decode_fast_kernel(const RnDecodeParams p) {
     extern __shared__ __align__(128) unsigned char row_bytes_buf[];  // per warp: K rows of C floats
     __shared__ int sel_slot[RN_DECF_PAIRS][2][K];
@@ -248,179 +334,190 @@ __global__ void __launch_bounds__(RN_DECF_THREADS, 2) rn_decode_fast_kernel(cons
         rn_mbar_fence_init();
     }
 
-    if (warp < 4) {
-        // four lanes per address: 32 addresses (16 pairs x write/read) on warps 0-3
-        const int group = tid >> 2, gl = tid & 3;
-        const int pair = group & 15, which = group >> 4;
-        const int bh = min(bh0 + pair, BH - 1);  // surplus groups redo the last pair and discard it
-        const int b = bh / p.H, h = bh % p.H;
-        const T *src = static_cast<const T *>(which ? p.r_addr : p.w_addr) + rn_in_row(p, bh, p.ld_addr[which ? 1 : 0], U * P);
-        int content[K];
-        float weight[K];
-        rn_fast::quad_decode<T, U, P, K>(src, p.re_norm[which], gl, content, weight);
-        if (gl == 0 && bh0 + pair < BH) {
-            const int shift = (h < p.E) ? rn_pos_mod(rn_pos_at(p.pos, b, 0), p.A) : 0;
-#pragma unroll
-            for (int e = 0; e < K; ++e) {
-                sel_slot[pair][which][e] = rn_cape(content[e], shift, p.A);
-                sel_val[pair][which][e] = weight[e];
-            }
-        }
-    }
-    __syncthreads();
-
     uint32_t phase = 0;  // parity of this warp's mbarrier
+    bool lost = false;   // a copy never landed: this warp leaves its pairs alone from then on
 #pragma unroll 1
-    for (int pp = 0; pp < 2; ++pp) {
-        const int pair = warp * 2 + pp;
-        const int bh = bh0 + pair;
-        if (bh >= BH) break;
-        const int b = bh / p.H;
-        T *y = static_cast<T *>(p.y) + int64_t(bh) * C;
-        if (p.mask != nullptr && p.mask[b] == 0) {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) rn_store4<T>(y + v * 128 + lane * 4, make_float4(0.f, 0.f, 0.f, 0.f));
-            continue;
+    for (int step = 0; step < (STEPS ? p.steps : 1); ++step) {
+        if (step > 0) {
+            rn_bulk_wait_all();  // the rows that the step before sent are there; the next ones are read by the same engine
+            rn_fence_proxy_async();
+            __syncthreads();     // its addresses have been read
         }
-        float *slot = p.slot + int64_t(bh) * p.A * C;
-        float *mass = p.mass + int64_t(bh) * p.A;
-        const float gamma = rn_to_float<T>(static_cast<const T *>(p.gamma)[rn_in_row(p, bh, p.ld_gamma, 1)]);
-        float4 xv[NV];
+        if (warp < 4) {
+            // four lanes per address: 32 addresses (16 pairs x write/read) on warps 0-3
+            const int group = tid >> 2, gl = tid & 3;
+            const int pair = group & 15, which = group >> 4;
+            const int bh = min(bh0 + pair, BH - 1);  // surplus groups redo the last pair and discard it
+            const int b = bh / p.H, h = bh % p.H;
+            const T *src = static_cast<const T *>(which ? p.r_addr : p.w_addr) + step * p.st_addr[which] + rn_in_row(p, bh, p.ld_addr[which], U * P);
+            int content[K];
+            float weight[K];
+            rn_fast::quad_decode<T, U, P, K>(src, p.re_norm[which], gl, content, weight);
+            if (gl == 0 && bh0 + pair < BH) {
+                const int shift = (h < p.E) ? rn_pos_mod(rn_pos_at(p.pos, b, 0) + step, p.A) : 0;
 #pragma unroll
-        for (int v = 0; v < NV; ++v) xv[v] = rn_load4<T>(static_cast<const T *>(p.x) + rn_in_row(p, bh, p.ld_x, C) + v * 128 + lane * 4);
-
-        // ---- write rows: bulk copies into this warp's buffer -------------------------------------------
-        const int a_l = lane < K ? sel_slot[pair][0][lane] : 0;
-        const float w_l = lane < K ? sel_val[pair][0][lane] : 0.f;
-        const bool live_w = lane < K && w_l != 0.f;
-        const int nlive = __popc(__ballot_sync(RN_FULL, live_w));
-        if (nlive > 0) {
-            if (lane == 0) rn_mbar_expect_tx(&mbar[warp], uint32_t(nlive) * ROW_BYTES);
-            __syncwarp();
-            if (live_w) rn_bulk_g2s(wbuf + lane * (NV * 128), slot + int64_t(a_l) * C, ROW_BYTES, &mbar[warp]);
-        }
-
-        // ---- read rows: per-lane loads into registers, in flight together with the bulk copies -------------
-        const int ar_l = lane < K ? sel_slot[pair][1][lane] : 0;
-        float r_l = lane < K ? sel_val[pair][1][lane] : 0.f;
-        float4 rows[K][NV];
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const int a = __shfl_sync(RN_FULL, ar_l, k);
-#pragma unroll
-            for (int v = 0; v < NV; ++v) rows[k][v] = *reinterpret_cast<const float4 *>(slot + int64_t(a) * C + v * 128 + lane * 4);
-        }
-        // a read row that this step also writes: index of that write row, else -1
-        int alias_l = -1;
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-            const int aw = __shfl_sync(RN_FULL, a_l, j);
-            const float ww = __shfl_sync(RN_FULL, w_l, j);
-            if (ww != 0.f && aw == ar_l) alias_l = j;
-        }
-        float gain_l = 0.f, mass_new = 0.f;
-        if (live_w) {
-            const RnGate g = rn_gate(w_l, gamma, mass[a_l], p.eps);
-            gain_l = g.gain;
-            mass_new = g.mass;
-        }
-        __syncwarp();
-
-        bool landed = true;
-        if (nlive > 0) {
-            landed = rn_mbar_wait_bounded(&mbar[warp], phase);
-            phase ^= 1u;
-        }
-        if (!__all_sync(RN_FULL, landed)) {
-            // A bulk copy never completed: report it through the status word, leave slot AND mass of this
-            // pair as they were, give the pairs this warp still owns a defined (zero) output and stop using
-            // the buffer (the copy may still land).
-            if (lane == 0) atomicMax(p.status, RN_STATUS_WAIT_TIMEOUT);
-            for (int rest = pp; rest < 2 && bh0 + warp * 2 + rest < BH; ++rest) {
-                T *yr = static_cast<T *>(p.y) + int64_t(bh0 + warp * 2 + rest) * C;
-#pragma unroll
-                for (int v = 0; v < NV; ++v) rn_store4<T>(yr + v * 128 + lane * 4, make_float4(0.f, 0.f, 0.f, 0.f));
-            }
-            break;
-        }
-        if (live_w) mass[a_l] = mass_new;  // only once the rows are here: slot and mass move together
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const float w = __shfl_sync(RN_FULL, w_l, k);
-            const float gain = __shfl_sync(RN_FULL, gain_l, k);
-            if (w != 0.f) {
-#pragma unroll
-                for (int v = 0; v < NV; ++v) {
-                    float4 *cell = reinterpret_cast<float4 *>(wbuf + k * (NV * 128) + v * 128 + lane * 4);
-                    float4 s = *cell;
-                    s.x = fmaf(gain, xv[v].x - s.x, s.x);
-                    s.y = fmaf(gain, xv[v].y - s.y, s.y);
-                    s.z = fmaf(gain, xv[v].z - s.z, s.z);
-                    s.w = fmaf(gain, xv[v].w - s.w, s.w);
-                    *cell = s;
+                for (int e = 0; e < K; ++e) {
+                    sel_slot[pair][which][e] = rn_cape(content[e], shift, p.A);
+                    sel_val[pair][which][e] = weight[e];
                 }
             }
         }
-        rn_fence_proxy_async();  // the updated rows are read by the bulk copy engine next
-        __syncwarp();
-        if (live_w) rn_bulk_s2g(slot + int64_t(a_l) * C, wbuf + lane * (NV * 128), ROW_BYTES);
-        rn_bulk_commit();
+        __syncthreads();
 
-        // ---- reads (after the writes of this step) ---------------------------------------------------
-        float4 acc[NV];
+#pragma unroll 1
+        for (int pp = 0; pp < 2; ++pp) {
+            const int pair = warp * 2 + pp;
+            const int bh = bh0 + pair;
+            if (bh >= BH) break;
+            const int b = bh / p.H;
+            T *y = static_cast<T *>(p.y) + step * p.st_y + int64_t(bh) * C;
+            if (lost || (p.mask != nullptr && p.mask[b] == 0)) {
 #pragma unroll
-        for (int v = 0; v < NV; ++v) acc[v] = make_float4(0.f, 0.f, 0.f, 0.f);
-        float scale = 1.f;
-        {
-            if (p.mass_aware) {
-                const float rm = (lane < K && r_l != 0.f) ? r_l * mass[ar_l] : 0.f;
-                const float sr = rn_warp_sum(lane < K ? r_l : 0.f), srm = rn_warp_sum(rm);
-                scale = sr / (srm + p.eps);
-                r_l = rm;
+                for (int v = 0; v < NV; ++v) rn_store4<T>(y + v * 128 + lane * 4, make_float4(0.f, 0.f, 0.f, 0.f));
+                continue;
             }
+            float *slot = p.slot + int64_t(bh) * p.A * C;
+            float *mass = p.mass + int64_t(bh) * p.A;
+            const float gamma = rn_to_float<T>(static_cast<const T *>(p.gamma)[step * p.st_gamma + rn_in_row(p, bh, p.ld_gamma, 1)]);
+            float4 xv[NV];
 #pragma unroll
-            for (int k = K - 1; k >= 0; --k) {
-                const float coef = __shfl_sync(RN_FULL, r_l, k);
-                const int al = __shfl_sync(RN_FULL, alias_l, k);
-                if (coef != 0.f) {
+            for (int v = 0; v < NV; ++v) xv[v] = rn_load4<T>(static_cast<const T *>(p.x) + step * p.st_x + rn_in_row(p, bh, p.ld_x, C) + v * 128 + lane * 4);
+
+            // ---- write rows: bulk copies into this warp's buffer -------------------------------------------
+            const int a_l = lane < K ? sel_slot[pair][0][lane] : 0;
+            const float w_l = lane < K ? sel_val[pair][0][lane] : 0.f;
+            const bool live_w = lane < K && w_l != 0.f;
+            const int nlive = __popc(__ballot_sync(RN_FULL, live_w));
+            if (nlive > 0) {
+                if (lane == 0) rn_mbar_expect_tx(&mbar[warp], uint32_t(nlive) * ROW_BYTES);
+                __syncwarp();
+                if (live_w) rn_bulk_g2s(wbuf + lane * (NV * 128), slot + int64_t(a_l) * C, ROW_BYTES, &mbar[warp]);
+            }
+
+            // ---- read rows: per-lane loads into registers, in flight together with the bulk copies -------------
+            // (from the L2: an earlier step's copies have gone past this SM's L1)
+            const int ar_l = lane < K ? sel_slot[pair][1][lane] : 0;
+            float r_l = lane < K ? sel_val[pair][1][lane] : 0.f;
+            float4 rows[K][NV];
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const int a = __shfl_sync(RN_FULL, ar_l, k);
+#pragma unroll
+                for (int v = 0; v < NV; ++v) rows[k][v] = __ldcg(reinterpret_cast<const float4 *>(slot + int64_t(a) * C + v * 128 + lane * 4));
+            }
+            // a read row that this step also writes: index of that write row, else -1
+            int alias_l = -1;
+#pragma unroll
+            for (int j = 0; j < K; ++j) {
+                const int aw = __shfl_sync(RN_FULL, a_l, j);
+                const float ww = __shfl_sync(RN_FULL, w_l, j);
+                if (ww != 0.f && aw == ar_l) alias_l = j;
+            }
+            float gain_l = 0.f, mass_new = 0.f;
+            if (live_w) {
+                const RnGate g = rn_gate(w_l, gamma, mass[a_l], p.eps);
+                gain_l = g.gain;
+                mass_new = g.mass;
+            }
+            __syncwarp();
+
+            bool landed = true;
+            if (nlive > 0) {
+                landed = rn_mbar_wait_bounded(&mbar[warp], phase);
+                phase ^= 1u;
+            }
+            if (!__all_sync(RN_FULL, landed)) {
+                // A bulk copy never completed: report it through the status word, leave slot AND mass of this
+                // pair as they were, give the pairs this warp still owns a defined (zero) output and stop using
+                // the buffer (the copy may still land).
+                if (lane == 0) atomicMax(p.status, RN_STATUS_WAIT_TIMEOUT);
+                for (int rest = pp; rest < 2 && bh0 + warp * 2 + rest < BH; ++rest) {
+                    T *yr = static_cast<T *>(p.y) + step * p.st_y + int64_t(bh0 + warp * 2 + rest) * C;
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) rn_store4<T>(yr + v * 128 + lane * 4, make_float4(0.f, 0.f, 0.f, 0.f));
+                }
+                lost = true;
+                break;
+            }
+            if (live_w) mass[a_l] = mass_new;  // only once the rows are here: slot and mass move together
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const float w = __shfl_sync(RN_FULL, w_l, k);
+                const float gain = __shfl_sync(RN_FULL, gain_l, k);
+                if (w != 0.f) {
 #pragma unroll
                     for (int v = 0; v < NV; ++v) {
-                        float4 s = rows[k][v];
-                        if (al >= 0) s = *reinterpret_cast<const float4 *>(wbuf + al * (NV * 128) + v * 128 + lane * 4);
-                        acc[v].x = fmaf(coef, s.x, acc[v].x);
-                        acc[v].y = fmaf(coef, s.y, acc[v].y);
-                        acc[v].z = fmaf(coef, s.z, acc[v].z);
-                        acc[v].w = fmaf(coef, s.w, acc[v].w);
+                        float4 *cell = reinterpret_cast<float4 *>(wbuf + k * (NV * 128) + v * 128 + lane * 4);
+                        float4 s = *cell;
+                        s.x = fmaf(gain, xv[v].x - s.x, s.x);
+                        s.y = fmaf(gain, xv[v].y - s.y, s.y);
+                        s.z = fmaf(gain, xv[v].z - s.z, s.z);
+                        s.w = fmaf(gain, xv[v].w - s.w, s.w);
+                        *cell = s;
                     }
                 }
             }
-        }
-        rn_bulk_wait_read();  // the buffer is free again once the outgoing copies have read it
-        __syncwarp();
-        float sq = 0.f;
+            rn_fence_proxy_async();  // the updated rows are read by the bulk copy engine next
+            __syncwarp();
+            if (live_w) rn_bulk_s2g(slot + int64_t(a_l) * C, wbuf + lane * (NV * 128), ROW_BYTES);
+            rn_bulk_commit();
+
+            // ---- reads (after the writes of this step) ---------------------------------------------------
+            float4 acc[NV];
 #pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            acc[v].x *= scale; acc[v].y *= scale; acc[v].z *= scale; acc[v].w *= scale;
-            sq += acc[v].x * acc[v].x + acc[v].y * acc[v].y + acc[v].z * acc[v].z + acc[v].w * acc[v].w;
-        }
-        if (p.norm_weight != nullptr) {
-            const float inv_rms = rsqrtf(rn_warp_sum(sq) / float(C) + p.norm_eps);
+            for (int v = 0; v < NV; ++v) acc[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+            float scale = 1.f;
+            {
+                if (p.mass_aware) {
+                    const float rm = (lane < K && r_l != 0.f) ? r_l * mass[ar_l] : 0.f;
+                    const float sr = rn_warp_sum(lane < K ? r_l : 0.f), srm = rn_warp_sum(rm);
+                    scale = sr / (srm + p.eps);
+                    r_l = rm;
+                }
+#pragma unroll
+                for (int k = K - 1; k >= 0; --k) {
+                    const float coef = __shfl_sync(RN_FULL, r_l, k);
+                    const int al = __shfl_sync(RN_FULL, alias_l, k);
+                    if (coef != 0.f) {
+#pragma unroll
+                        for (int v = 0; v < NV; ++v) {
+                            float4 s = rows[k][v];
+                            if (al >= 0) s = *reinterpret_cast<const float4 *>(wbuf + al * (NV * 128) + v * 128 + lane * 4);
+                            acc[v].x = fmaf(coef, s.x, acc[v].x);
+                            acc[v].y = fmaf(coef, s.y, acc[v].y);
+                            acc[v].z = fmaf(coef, s.z, acc[v].z);
+                            acc[v].w = fmaf(coef, s.w, acc[v].w);
+                        }
+                    }
+                }
+            }
+            rn_bulk_wait_read();  // the buffer is free again once the outgoing copies have read it
+            __syncwarp();
+            float sq = 0.f;
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
-                const float4 nw = *reinterpret_cast<const float4 *>(p.norm_weight + v * 128 + lane * 4);
-                acc[v].x *= inv_rms * nw.x; acc[v].y *= inv_rms * nw.y; acc[v].z *= inv_rms * nw.z; acc[v].w *= inv_rms * nw.w;
+                acc[v].x *= scale; acc[v].y *= scale; acc[v].z *= scale; acc[v].w *= scale;
+                sq += acc[v].x * acc[v].x + acc[v].y * acc[v].y + acc[v].z * acc[v].z + acc[v].w * acc[v].w;
             }
-        }
-        if (p.gate != nullptr) {
+            if (p.norm_weight != nullptr) {
+                const float inv_rms = rsqrtf(rn_warp_sum(sq) / float(C) + p.norm_eps);
 #pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                const float4 gl = rn_load4<T>(static_cast<const T *>(p.gate) + rn_in_row(p, bh, p.ld_gate, C) + v * 128 + lane * 4);
-                acc[v].x /= 1.f + expf(-gl.x); acc[v].y /= 1.f + expf(-gl.y);
-                acc[v].z /= 1.f + expf(-gl.z); acc[v].w /= 1.f + expf(-gl.w);
+                for (int v = 0; v < NV; ++v) {
+                    const float4 nw = *reinterpret_cast<const float4 *>(p.norm_weight + v * 128 + lane * 4);
+                    acc[v].x *= inv_rms * nw.x; acc[v].y *= inv_rms * nw.y; acc[v].z *= inv_rms * nw.z; acc[v].w *= inv_rms * nw.w;
+                }
             }
-        }
+            if (p.gate != nullptr) {
 #pragma unroll
-        for (int v = 0; v < NV; ++v) rn_store4<T>(y + v * 128 + lane * 4, acc[v]);
+                for (int v = 0; v < NV; ++v) {
+                    const float4 gl = rn_load4<T>(static_cast<const T *>(p.gate) + step * p.st_gate + rn_in_row(p, bh, p.ld_gate, C) + v * 128 + lane * 4);
+                    acc[v].x /= 1.f + expf(-gl.x); acc[v].y /= 1.f + expf(-gl.y);
+                    acc[v].z /= 1.f + expf(-gl.z); acc[v].w /= 1.f + expf(-gl.w);
+                }
+            }
+#pragma unroll
+            for (int v = 0; v < NV; ++v) rn_store4<T>(y + v * 128 + lane * 4, acc[v]);
+        }
     }
 }
 
@@ -717,6 +814,256 @@ __device__ __forceinline__ uint32_t rn_decode_pair_task(const RnDecodeParams &p,
     return phase;
 }
 
+// ------------------------------------------------------------------------------------------
+// several steps of one launch, the shapes of the kernel above: a pair of warps per (b,h) pair
+// ------------------------------------------------------------------------------------------
+// What bounds a step of one pair is a chain of latencies (decode the addresses, fetch the rows, send them back), so one warp
+// decodes the addresses of step i + 1 while the other moves the rows of step i; the write and the read rows of a step
+// are fetched together, into two buffers.  One barrier of the two warps per step hands the addresses over.  Thirteen
+// pairs of warps fill the shared memory of an SM at C = 128, six at C = 256.  16 steps at 64 x 16 pairs, C = 128: 154 us with
+// the single-step kernel's loop over steps (decode and two fetches one after the other), 227 us as sixteen launches.
+template <int NV> struct RnDecSteps { static constexpr int PAIRS = NV == 1 ? 13 : 6, THREADS = PAIRS * 64; };
+
+template <typename T, int NV, bool EXTRA>
+__global__ void __launch_bounds__(RnDecSteps<NV>::THREADS, 1) rn_decode_steps_kernel(const RnDecodeParams p) {
+    constexpr int RN_DECS_PAIRS = RnDecSteps<NV>::PAIRS;
+    constexpr int U = 2, P = 64, K = 16, C = NV * 128;
+    constexpr uint32_t ROW_BYTES = C * 4;
+    extern __shared__ __align__(128) unsigned char row_bytes_buf[];  // per row warp: K write rows, K read rows of C floats
+    __shared__ __align__(8) uint64_t mbar[RN_DECS_PAIRS];
+    __shared__ int sel_slot[RN_DECS_PAIRS][2][32];                   // by parity of the step; lanes 0-15 write, 16-31 read
+    __shared__ float sel_val[RN_DECS_PAIRS][2][32];
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int w = warp % RN_DECS_PAIRS;
+    const int BH = p.B * p.H, n = p.steps;
+    const int first = int(int64_t(BH) * blockIdx.x / gridDim.x), last = int(int64_t(BH) * (blockIdx.x + 1) / gridDim.x);
+    const int mine = first + w < last ? (last - first - w + RN_DECS_PAIRS - 1) / RN_DECS_PAIRS : 0;
+    if (tid < RN_DECS_PAIRS) {
+        rn_mbar_init(&mbar[tid], 1);
+        rn_mbar_fence_init();
+    }
+    __syncthreads();
+    auto meet = [w] { asm volatile("bar.sync %0, 64;" ::"r"(w + 1) : "memory"); };
+
+    if (warp >= RN_DECS_PAIRS) {
+        // ================================ addresses =========================================================
+        const uint32_t cand = rn_half::load_candidates(lane & 15);
+        const int which = lane >> 4;
+        const T *base = static_cast<const T *>(which ? p.r_addr : p.w_addr);
+        int i = 0;
+#pragma unroll 1
+        for (int turn = 0; turn < mine; ++turn) {
+            const int bh = first + w + turn * RN_DECS_PAIRS, b = bh / p.H, h = bh - b * p.H;
+            const T *src = base + (EXTRA ? rn_in_row(p, bh, p.ld_addr[which], U * P) : int64_t(bh) * (U * P));
+            const int pos = h < p.E ? rn_pos_at(p.pos, b, 0) : 0;
+            uint2 next[2];
+            rn_half::load_logits<T>(src, lane, next);
+#pragma unroll 1
+            for (int step = 0; step < n; ++step, ++i) {
+                const uint2 logits[2] = {next[0], next[1]};
+                if (step + 1 < n) rn_half::load_logits<T>(src + (step + 1) * p.st_addr[which], lane, next);
+                int content;
+                float weight;
+                rn_half::decode_u2p64k16<T>(logits, p.re_norm[which], lane, cand, content, weight);
+                sel_slot[w][i & 1][lane] = rn_cape(content, h < p.E ? rn_pos_mod(pos + step, p.A) : 0, p.A);
+                sel_val[w][i & 1][lane] = weight;
+                meet();  // step i is there; the rows of step i - 1 are done with its addresses
+            }
+        }
+        return;
+    }
+
+    // ================================ rows ==================================================================
+    float *wbuf = reinterpret_cast<float *>(row_bytes_buf) + size_t(w) * 2 * K * C, *rbuf = wbuf + K * C;
+    const T *in_x = static_cast<const T *>(p.x), *in_gamma = static_cast<const T *>(p.gamma), *in_gate = static_cast<const T *>(p.gate);
+    uint32_t phase = 0;
+    bool lost = false;  // a copy never landed: nothing but zeros from then on
+    int i = 0;
+#pragma unroll 1
+    for (int turn = 0; turn < mine; ++turn) {
+        const int bh = first + w + turn * RN_DECS_PAIRS, b = bh / p.H;
+        const bool off = p.mask != nullptr && p.mask[b] == 0;
+        float *slot = p.slot + int64_t(bh) * p.A * C;
+        float *mass = p.mass + int64_t(bh) * p.A;
+        const int64_t at_x = EXTRA ? rn_in_row(p, bh, p.ld_x, C) : int64_t(bh) * C;
+        const int64_t at_gate = EXTRA ? rn_in_row(p, bh, p.ld_gate, C) : int64_t(bh) * C;
+        const int64_t at_gamma = EXTRA ? rn_in_row(p, bh, p.ld_gamma, 1) : int64_t(bh);
+#pragma unroll 1
+        for (int step = 0; step < n; ++step, ++i) {
+            T *y = static_cast<T *>(p.y) + step * p.st_y + int64_t(bh) * C + lane * 4;
+            RnRaw4<T> xraw[NV];
+            const float gamma = rn_to_float<T>(in_gamma[step * p.st_gamma + at_gamma]);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) xraw[v] = rn_load_raw4<T>(in_x + step * p.st_x + at_x + v * 128 + lane * 4);
+            meet();
+            if (off || lost) {
+#pragma unroll
+                for (int v = 0; v < NV; ++v) rn_store4<T>(y + v * 128, make_float4(0.f, 0.f, 0.f, 0.f));
+                continue;
+            }
+            const int my_slot = sel_slot[w][i & 1][lane];
+            const float weight = sel_val[w][i & 1][lane];
+            const bool live = weight != 0.f, live_w = live && lane < K;
+            // a read row that this step also writes is taken from the updated copy: one match finds the equal slots
+            const unsigned live_mask = __ballot_sync(RN_FULL, live_w);
+            const unsigned same = __match_any_sync(RN_FULL, my_slot) & live_mask;
+            const int alias_l = same ? __ffs(same) - 1 : -1;
+            const bool want = lane < K ? live_w : live && alias_l < 0;
+            const unsigned rows = __ballot_sync(RN_FULL, want);
+            rn_bulk_wait_all();      // the rows that the step before sent are there (and its masses, by the barrier)
+            rn_fence_proxy_async();
+            __syncwarp();
+            bool landed = true;
+            if (rows != 0u) {
+                if (lane == 0) rn_mbar_expect_tx(&mbar[w], uint32_t(__popc(rows)) * ROW_BYTES);
+                __syncwarp();
+                if (want) rn_bulk_g2s(wbuf + lane * C, slot + int64_t(my_slot) * C, ROW_BYTES, &mbar[w]);
+            }
+            const float mass_l = live_w ? mass[my_slot] : 0.f;
+            float coef_l = weight, mass_new = 0.f;  // lanes 0-15: gain of a write row; 16-31: weight of a read row
+            if (live_w) {
+                const RnGate g = rn_gate(weight, gamma, mass_l, p.eps);
+                coef_l = g.gain;
+                mass_new = g.mass;
+            }
+            if (rows != 0u) {
+                landed = rn_mbar_wait_bounded(&mbar[w], phase);
+                phase ^= 1u;
+            }
+            if (!__all_sync(RN_FULL, landed)) {
+                // reported through the status word; slot and mass stay as the step before left them, and the buffers are not
+                // used again (the copy may still land)
+                if (lane == 0) atomicMax(p.status, RN_STATUS_WAIT_TIMEOUT);
+                lost = true;
+#pragma unroll
+                for (int v = 0; v < NV; ++v) rn_store4<T>(y + v * 128, make_float4(0.f, 0.f, 0.f, 0.f));
+                continue;
+            }
+            if (live_w) mass[my_slot] = mass_new;  // only once the rows are here: slot and mass move together
+            float4 xv[NV], acc[NV];
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                xv[v] = rn_cvt_raw4(xraw[v]);
+                acc[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int k0 = 0; k0 < K; k0 += 4) {
+                float4 cur[4][NV];
+                float gain[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    gain[q] = __shfl_sync(RN_FULL, coef_l, k0 + q);
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) cur[q][v] = *reinterpret_cast<const float4 *>(wbuf + (k0 + q) * C + v * 128 + lane * 4);
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (!(rows & (1u << (k0 + q)))) continue;  // not loaded: the buffer holds stale rows there
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) {
+                        float4 s = cur[q][v];
+                        s.x = fmaf(gain[q], xv[v].x - s.x, s.x);
+                        s.y = fmaf(gain[q], xv[v].y - s.y, s.y);
+                        s.z = fmaf(gain[q], xv[v].z - s.z, s.z);
+                        s.w = fmaf(gain[q], xv[v].w - s.w, s.w);
+                        *reinterpret_cast<float4 *>(wbuf + (k0 + q) * C + v * 128 + lane * 4) = s;
+                    }
+                }
+            }
+            rn_fence_proxy_async();  // the updated rows are read by the bulk copy engine next
+            __syncwarp();
+            if (live_w) rn_bulk_s2g(slot + int64_t(my_slot) * C, wbuf + lane * C, ROW_BYTES);
+            rn_bulk_commit();
+
+            // ---- reads, after the writes of this step: first the rows that it wrote, then the others ----------------
+            float scale = 1.f;
+            if (p.mass_aware) {
+                const float r = lane < K ? 0.f : weight;
+                const float rm = r != 0.f ? r * mass[my_slot] : 0.f;
+                const float sr = rn_warp_sum(r), srm = rn_warp_sum(rm);
+                scale = sr / (srm + p.eps);
+                if (lane >= K) coef_l = rm;
+            }
+            const bool live_r = lane >= K && coef_l != 0.f;
+            const unsigned from_w = __ballot_sync(RN_FULL, live_r && alias_l >= 0) >> 16, from_r = __ballot_sync(RN_FULL, live_r && alias_l < 0) >> 16;
+            if (from_w != 0u) {      // rare
+#pragma unroll 1
+                for (int k = 0; k < K; ++k) {
+                    const float coef = __shfl_sync(RN_FULL, coef_l, K + k);
+                    const int al = __shfl_sync(RN_FULL, alias_l, K + k);
+                    if (from_w >> k & 1u) {
+#pragma unroll
+                        for (int v = 0; v < NV; ++v) {
+                            const float4 s = *reinterpret_cast<const float4 *>(wbuf + al * C + v * 128 + lane * 4);
+                            acc[v].x = fmaf(coef, s.x, acc[v].x);
+                            acc[v].y = fmaf(coef, s.y, acc[v].y);
+                            acc[v].z = fmaf(coef, s.z, acc[v].z);
+                            acc[v].w = fmaf(coef, s.w, acc[v].w);
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int k0 = 0; k0 < K; k0 += 4) {
+                float4 cur[4][NV];
+                float coef[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    coef[q] = __shfl_sync(RN_FULL, coef_l, K + k0 + q);
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) cur[q][v] = *reinterpret_cast<const float4 *>(rbuf + (k0 + q) * C + v * 128 + lane * 4);
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (!(from_r & (1u << (k0 + q)))) continue;
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) {
+                        acc[v].x = fmaf(coef[q], cur[q][v].x, acc[v].x);
+                        acc[v].y = fmaf(coef[q], cur[q][v].y, acc[v].y);
+                        acc[v].z = fmaf(coef[q], cur[q][v].z, acc[v].z);
+                        acc[v].w = fmaf(coef[q], cur[q][v].w, acc[v].w);
+                    }
+                }
+            }
+            float sq = 0.f;
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                acc[v].x *= scale; acc[v].y *= scale; acc[v].z *= scale; acc[v].w *= scale;
+                sq += acc[v].x * acc[v].x + acc[v].y * acc[v].y + acc[v].z * acc[v].z + acc[v].w * acc[v].w;
+            }
+            if (p.norm_weight != nullptr) {
+                const float inv_rms = rsqrtf(rn_warp_sum(sq) / float(C) + p.norm_eps);
+#pragma unroll
+                for (int v = 0; v < NV; ++v) {
+                    const float4 nw = *reinterpret_cast<const float4 *>(p.norm_weight + v * 128 + lane * 4);
+                    acc[v].x *= inv_rms * nw.x; acc[v].y *= inv_rms * nw.y; acc[v].z *= inv_rms * nw.z; acc[v].w *= inv_rms * nw.w;
+                }
+            }
+            if (in_gate != nullptr) {
+#pragma unroll
+                for (int v = 0; v < NV; ++v) {
+                    const float4 gl = rn_load4<T>(in_gate + step * p.st_gate + at_gate + v * 128 + lane * 4);
+                    acc[v].x /= 1.f + expf(-gl.x); acc[v].y /= 1.f + expf(-gl.y);
+                    acc[v].z /= 1.f + expf(-gl.z); acc[v].w /= 1.f + expf(-gl.w);
+                }
+            }
+#pragma unroll
+            for (int v = 0; v < NV; ++v) rn_store4<T>(y + v * 128, acc[v]);
+        }
+    }
+    rn_bulk_wait_read();  // the buffers go away with the block
+}
+
+template <typename T, int NV, bool EXTRA>
+static int rn_launch_decode_steps(const RnDecodeParams &p, int sms, cudaStream_t stream) {
+    constexpr int smem = RnDecSteps<NV>::PAIRS * 2 * 16 * NV * 128 * 4;
+    if (cudaFuncSetAttribute(rn_decode_steps_kernel<T, NV, EXTRA>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -1;
+    const int pairs = p.B * p.H;
+    rn_decode_steps_kernel<T, NV, EXTRA><<<pairs < sms ? pairs : sms, RnDecSteps<NV>::THREADS, smem, stream>>>(p);
+    return 0;
+}
+
 // 0 = launched, -1 = not this kernel's shape
 template <typename T>
 static int rn_launch_decode_pair(const RnDecodeParams &p, int device, cudaStream_t stream) {
@@ -728,6 +1075,12 @@ static int rn_launch_decode_pair(const RnDecodeParams &p, int device, cudaStream
         const int threads = p.C == 128 ? RnDecPair<1>::THREADS : RnDecPair<2>::THREADS;
         const bool extra = p.scale[0] != nullptr || p.ld_addr[0] != int64_t(p.H) * p.U * p.P || p.ld_addr[1] != int64_t(p.H) * p.U * p.P ||
                            p.ld_x != int64_t(p.H) * p.C || p.ld_gamma != p.H || (p.gate != nullptr && p.ld_gate != int64_t(p.H) * p.C);
+        if (p.steps > 1) {
+            if (p.scale[0] != nullptr) return -1;
+            const int sms = rn_sm_count(device);
+            if (p.C == 128) return extra ? rn_launch_decode_steps<T, 1, true>(p, sms, stream) : rn_launch_decode_steps<T, 1, false>(p, sms, stream);
+            return extra ? rn_launch_decode_steps<T, 2, true>(p, sms, stream) : rn_launch_decode_steps<T, 2, false>(p, sms, stream);
+        }
         const int wpc = threads / 32;
         // CTAs: enough for one warp per pair, but at least one per SM while there are pairs to hand out (a small
         // batch is spread over all SMs instead of filling a few), at most the two resident CTAs per SM
@@ -758,24 +1111,21 @@ static int rn_launch_decode_pair(const RnDecodeParams &p, int device, cudaStream
     }
 }
 
+template <typename T, int U, int P, int K, int NV, bool STEPS>
+static int rn_launch_decode_fast_s(const RnDecodeParams &p, cudaStream_t stream) {
+    const int grid = (p.B * p.H + RN_DECF_PAIRS - 1) / RN_DECF_PAIRS;
+    constexpr int smem = (RN_DECF_THREADS / 32) * K * NV * 128 * 4;  // one buffer of K rows per warp
+    if (cudaFuncSetAttribute(rn_decode_fast_kernel<T, U, P, K, NV, STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        return -1;
+    rn_decode_fast_kernel<T, U, P, K, NV, STEPS><<<grid, RN_DECF_THREADS, smem, stream>>>(p);
+    return 0;
+}
+
 template <typename T, int U, int P, int K>
 static int rn_launch_decode_fast_c(const RnDecodeParams &p, cudaStream_t stream) {
-    const int grid = (p.B * p.H + RN_DECF_PAIRS - 1) / RN_DECF_PAIRS;
-    // dynamic shared memory: one buffer of K rows per warp
-    if (p.C == 128) {
-        constexpr int smem = (RN_DECF_THREADS / 32) * K * 128 * 4;
-        if (cudaFuncSetAttribute(rn_decode_fast_kernel<T, U, P, K, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-            return -1;
-        rn_decode_fast_kernel<T, U, P, K, 1><<<grid, RN_DECF_THREADS, smem, stream>>>(p);
-    } else if (p.C == 256) {
-        constexpr int smem = (RN_DECF_THREADS / 32) * K * 256 * 4;
-        if (cudaFuncSetAttribute(rn_decode_fast_kernel<T, U, P, K, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-            return -1;
-        rn_decode_fast_kernel<T, U, P, K, 2><<<grid, RN_DECF_THREADS, smem, stream>>>(p);
-    } else {
-        return -1;
-    }
-    return 0;
+    if (p.C == 128) return p.steps > 1 ? rn_launch_decode_fast_s<T, U, P, K, 1, true>(p, stream) : rn_launch_decode_fast_s<T, U, P, K, 1, false>(p, stream);
+    if (p.C == 256) return p.steps > 1 ? rn_launch_decode_fast_s<T, U, P, K, 2, true>(p, stream) : rn_launch_decode_fast_s<T, U, P, K, 2, false>(p, stream);
+    return -1;
 }
 
 // 0 = launched, -1 = no specialised kernel for this shape
@@ -787,7 +1137,7 @@ static int rn_launch_decode_fast(const RnDecodeParams &p, int device, cudaStream
                          reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.y) |
                          reinterpret_cast<uintptr_t>(p.gate) | reinterpret_cast<uintptr_t>(p.norm_weight);
     if ((io & 15) != 0 || (size_t(p.U) * p.P * esz) % 16 != 0) return -1;
-    if (((p.ld_addr[0] | p.ld_addr[1] | p.ld_x | p.ld_gate) * int64_t(esz)) % 16 != 0) return -1;
+    if (((p.ld_addr[0] | p.ld_addr[1] | p.ld_x | p.ld_gate | p.st_addr[0] | p.st_addr[1] | p.st_x | p.st_gate) * int64_t(esz)) % 16 != 0) return -1;
     if (rn_launch_decode_pair<T>(p, device, stream) == 0) return 0;
     if (p.U == 2 && p.P == 64 && p.K[0] == 16) return rn_launch_decode_fast_c<T, 2, 64, 16>(p, stream);
     if (p.U == 3 && p.P == 32 && p.K[0] == 8) return rn_launch_decode_fast_c<T, 3, 32, 8>(p, stream);
@@ -801,7 +1151,7 @@ template <typename T>
 static int rn_launch_decode(const RnDecodeParams &p, int kpl, int ppl, int grid, size_t smem, cudaStream_t stream) {
 #define RN_CASE(KP, PP)                                                                       \
     if (kpl == KP && ppl == PP) {                                                             \
-        rn_decode_kernel<T, KP, PP><<<grid, RN_DEC_WARPS * 32, smem, stream>>>(p);            \
+        rn_decode_kernel<T, KP, PP><<<grid, RN_DEC_THREADS, smem, stream>>>(p);            \
         return 0;                                                                             \
     }
     RN_CASE(1, 1) RN_CASE(1, 2) RN_CASE(1, 4) RN_CASE(2, 1) RN_CASE(2, 2) RN_CASE(2, 4) RN_CASE(4, 1) RN_CASE(4, 2)
@@ -843,7 +1193,21 @@ extern "C" int rn_decode_step_pos(const void *w_addr, const void *r_addr, const 
                                   double norm_eps, const void *w_scale, const void *r_scale, const int64_t *batch_strides,
                                   int64_t B, int64_t H, int64_t U, int64_t P, int64_t C, int64_t E, int64_t Kw, int64_t Kr,
                                   double w_re_norm, double r_re_norm, int mass_aware, double eps, int device, void *stream) {
+    return rn_decode_steps(w_addr, r_addr, x, gamma, dtype, slot, mass, mask, pos, pos_kind, pos_stride, y, norm_weight, gate_logits,
+                           norm_eps, w_scale, r_scale, batch_strides, 1, nullptr, B, H, U, P, C, E, Kw, Kr, w_re_norm, r_re_norm,
+                           mass_aware, eps, device, stream);
+}
+
+extern "C" int rn_decode_steps(const void *w_addr, const void *r_addr, const void *x, const void *gamma, int dtype,
+                               float *slot, float *mass, const uint8_t *mask, const void *pos, int pos_kind,
+                               int64_t pos_stride, void *y, const float *norm_weight, const void *gate_logits,
+                               double norm_eps, const void *w_scale, const void *r_scale, const int64_t *batch_strides,
+                               int64_t steps, const int64_t *step_strides, int64_t B, int64_t H, int64_t U, int64_t P,
+                               int64_t C, int64_t E, int64_t Kw, int64_t Kr, double w_re_norm, double r_re_norm,
+                               int mass_aware, double eps, int device, void *stream) {
     rn_clear_error();
+    RN_REQUIRE(steps == 1 || w_scale == nullptr, "logit scales are for a single step");
+    RN_REQUIRE(steps > 0 && steps < (int64_t(1) << 30) && (steps == 1 || step_strides != nullptr), "several steps need their strides");
     RN_REQUIRE(pos_kind >= RN_POS_I32 && pos_kind <= RN_POS_INDEX, "unknown kind of positions: %d", pos_kind);
     RN_REQUIRE((w_scale == nullptr) == (r_scale == nullptr), "give both logit scales or none");
     RN_REQUIRE(w_scale == nullptr || rn_decode_scales_supported(dtype, U, P, C, Kw, Kr),
@@ -882,6 +1246,12 @@ extern "C" int rn_decode_step_pos(const void *w_addr, const void *r_addr, const 
     p.ld_gate = batch_strides ? batch_strides[4] : H * C;
     RN_REQUIRE(p.ld_addr[0] >= H * U * P && p.ld_addr[1] >= H * U * P && p.ld_x >= H * C && p.ld_gamma >= H && p.ld_gate >= H * C,
                "a batch stride is smaller than a batch row");
+    p.steps = int(steps);
+    if (steps > 1) {
+        p.st_addr[0] = step_strides[0]; p.st_addr[1] = step_strides[1]; p.st_x = step_strides[2]; p.st_gamma = step_strides[3];
+        p.st_gate = step_strides[4];
+        p.st_y = B * H * C;
+    }
     p.B = int(B); p.H = int(H); p.U = int(U); p.P = int(P); p.C = int(C); p.E = int(E); p.A = int(A);
     p.K[0] = int(Kw); p.K[1] = int(Kr);
     p.re_norm[0] = float(w_re_norm); p.re_norm[1] = float(r_re_norm);
@@ -890,7 +1260,7 @@ extern "C" int rn_decode_step_pos(const void *w_addr, const void *r_addr, const 
     RN_REQUIRE(p.status != nullptr, "cannot locate the status word of device %d", device);
 
     const int kpl = rn_per_lane_dec(Kw > Kr ? Kw : Kr), ppl = rn_per_lane_dec(P);
-    const size_t smem = size_t(C) * (1 + RN_DEC_WARPS) * sizeof(float);
+    const size_t smem = size_t(C) * (2 + RN_DEC_WARPS) * sizeof(float);
     const int grid = int(B * H);
     int rc;
     rn_prof_reset();

@@ -216,6 +216,15 @@ def decode_scales_supported(dtype, U, P, C, w_top_k, r_top_k) -> bool:
     return code is not None and bool(lib.rn_decode_scales_supported(code, U, P, C, w_top_k, r_top_k))
 
 
+def _check_decode_state(slot, mass, shape):
+    if slot.dtype != torch.float32 or mass.dtype != torch.float32:
+        raise RuntimeError(f"slot/mass state must be float32, got {slot.dtype}/{mass.dtype}")
+    if not (slot.is_contiguous() and mass.is_contiguous()):
+        raise RuntimeError("Tensor slot/mass must be contiguous")
+    if tuple(slot.shape) != shape or tuple(mass.shape) != shape[:3]:
+        raise RuntimeError(f"state shape mismatch: slot {tuple(slot.shape)}, mass {tuple(mass.shape)}")
+
+
 def decode_impl(w_addr, r_addr, x, gamma, slot, mass, mask, embed_num, position_ids, w_top_k, r_top_k, w_re_norm,
                 r_re_norm, mass_aware, eps, norm_weight=None, gate_logits=None, norm_eps=0.0, w_scale=None, r_scale=None):
     """One decode step.  ``w_scale`` / ``r_scale`` (H,U) or (H,U,1): factors of the logits, applied inside the
@@ -223,12 +232,7 @@ def decode_impl(w_addr, r_addr, x, gamma, slot, mass, mask, embed_num, position_
     _require_cuda(w_addr, r_addr, x, gamma, slot, mass, position_ids)
     B, H, U, P = w_addr.shape
     C = x.shape[-1]
-    if slot.dtype != torch.float32 or mass.dtype != torch.float32:
-        raise RuntimeError(f"slot/mass state must be float32, got {slot.dtype}/{mass.dtype}")
-    if not (slot.is_contiguous() and mass.is_contiguous()):
-        raise RuntimeError("Tensor slot/mass must be contiguous")
-    if tuple(slot.shape) != (B, H, P ** U, C) or tuple(mass.shape) != (B, H, P ** U):
-        raise RuntimeError(f"state shape mismatch: slot {tuple(slot.shape)}, mass {tuple(mass.shape)}")
+    _check_decode_state(slot, mass, (B, H, P ** U, C))
     if (w_scale is None) != (r_scale is None):
         raise RuntimeError("give both logit scales or none")
     if w_scale is not None:
@@ -258,6 +262,44 @@ def decode_impl(w_addr, r_addr, x, gamma, slot, mass, mask, embed_num, position_
                                     ptr(w_scale), ptr(r_scale), batch_strides, B, H, U, P, C, embed_num, w_top_k, r_top_k,
                                     float(w_re_norm), float(r_re_norm), int(mass_aware), float(eps), x.device.index,
                                     stream_of(x)))
+    check_device(y)
+    return y
+
+
+def _step_rows(t: torch.Tensor) -> torch.Tensor:
+    """Inputs of several steps, (steps, B, ...): every batch row one contiguous block, any stride between rows and steps."""
+    return t if t[0].numel() == 0 or _batch_rows(t[0]).data_ptr() == t.data_ptr() else t.contiguous()
+
+
+def decode_steps_impl(w_addr, r_addr, x, gamma, slot, mass, mask, embed_num, position_ids, w_top_k, r_top_k, w_re_norm,
+                      r_re_norm, mass_aware, eps, norm_weight=None, gate_logits=None, norm_eps=0.0):
+    """Consecutive decode steps, inputs (steps, B, ...), in one launch; step j runs at ``position_ids + j``, which is left
+    as it is.  Returns (steps, B, H, C)."""
+    _require_cuda(w_addr, r_addr, x, gamma, slot, mass, position_ids)
+    steps, B, H, U, P = w_addr.shape
+    C = x.shape[-1]
+    _check_decode_state(slot, mass, (B, H, P ** U, C))
+    w_addr, r_addr, x, gamma = (_step_rows(t) for t in (w_addr, r_addr, x, gamma))
+    if not (r_addr.dtype == x.dtype == gamma.dtype == w_addr.dtype):
+        raise RuntimeError("w_addr, r_addr, x and gamma must share one dtype")
+    pos = _int32(position_ids).contiguous()
+    mask_u8 = None
+    if mask is not None and mask.numel() > 0:
+        mask_u8 = mask.to(torch.bool).contiguous().view(torch.uint8)
+    if norm_weight is not None:
+        norm_weight = norm_weight.to(torch.float32).contiguous()
+    if gate_logits is not None:
+        gate_logits = _step_rows(gate_logits.to(x.dtype))
+    y = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+    if y.numel() == 0:
+        return y
+    inputs = (w_addr, r_addr, x, gamma, x if gate_logits is None else gate_logits)
+    batch_strides = (ctypes.c_int64 * 5)(*(t.stride(1) for t in inputs))
+    step_strides = (ctypes.c_int64 * 5)(*(t.stride(0) for t in inputs))
+    check(lib.rn_decode_steps(ptr(w_addr), ptr(r_addr), ptr(x), ptr(gamma), dtype_code(x), ptr(slot), ptr(mass), ptr(mask_u8),
+                              ptr(pos), 0, 1, ptr(y), ptr(norm_weight), ptr(gate_logits), float(norm_eps), None, None,
+                              batch_strides, steps, step_strides, B, H, U, P, C, embed_num, w_top_k, r_top_k,
+                              float(w_re_norm), float(r_re_norm), int(mass_aware), float(eps), x.device.index, stream_of(x)))
     check_device(y)
     return y
 

@@ -2,8 +2,9 @@
 
 One autoregressive step of the slot memory is a single small kernel (tens of microseconds); launched
 from Python the host cost of a step is of the same size, so a generation loop is host bound.  This
-module captures ``n`` consecutive steps -- the fused decode operator on static input buffers plus the
-on-device increment of the position counter -- into one CUDA graph that is replayed with one launch.
+module captures ``n`` consecutive steps on static input buffers -- one launch of the decode kernel, whose thread groups
+go through the steps of the (batch, head) pairs they own, plus the on-device advance of the position counter -- into one
+CUDA graph that is replayed with one launch.
 
 It plays the role of the static-state decode loop of the reference's cache
 (packages/ramnet/src/ramnet/layers/cache.py:33-50,123-130: ``RAMCache.update`` keeps ``slot``/``mass`` and a
@@ -30,7 +31,7 @@ class DecodeGraph:
       ``gamma``               (n, B, H)         forget gate values, as the operator takes them
       ``gate_logits``         (n, B, H, C)      optional: sigmoid gate of the fused epilogue
     State updated in place by every replay: ``slot`` (B, H, A, C) fp32, ``mass`` (B, H, A) fp32 and
-    ``position_ids`` (B,) int32, which is advanced by one after every step.
+    ``position_ids`` (B,) int32, which is advanced by one for every step.
     ``outputs[j]`` is the (B, H, C) result of step ``j`` of the latest replay.
     """
 
@@ -56,37 +57,29 @@ class DecodeGraph:
         self.outputs: List[torch.Tensor] = []
         self._mask = mask if mask is not None else torch.empty(0, dtype=torch.bool, device=w_addr.device)
         rk = top_k if read_top_k is None else read_top_k
-        fused = norm_weight is not None or gate_logits is not None
-        ops = torch.ops.ramnet_ops
-
-        def step(j: int, bsel=slice(None), state=None) -> torch.Tensor:
+        def steps(bsel=slice(None), state=None) -> torch.Tensor:
             sl, ms, pos = state if state is not None else (slot, mass, position_ids)
             msk = self._mask if self._mask.numel() == 0 else self._mask[bsel]
-            if fused:
-                y = ops.decode_fused_(w_addr[j][bsel], r_addr[j][bsel], x[j][bsel], gamma[j][bsel], sl, ms, msk,
-                                      embed_num, pos, top_k, rk, w_re_norm, r_re_norm, mass_aware, eps, norm_weight,
-                                      None if gate_logits is None else gate_logits[j][bsel], norm_eps)
-            else:
-                y = ops.topk_autoregressive_(w_addr[j][bsel], r_addr[j][bsel], x[j][bsel], gamma[j][bsel], sl, ms, msk,
-                                             embed_num, pos, top_k, rk, w_re_norm, r_re_norm, mass_aware, eps)
-            pos.add_(1)
+            y = _ops.decode_steps_impl(w_addr[:, bsel], r_addr[:, bsel], x[:, bsel], gamma[:, bsel], sl, ms, msk, embed_num, pos,
+                                       top_k, rk, w_re_norm, r_re_norm, mass_aware, eps, norm_weight,
+                                       None if gate_logits is None else gate_logits[:, bsel], norm_eps)
+            pos.add_(n)
             return y
 
         # Warm-up on a side stream (lazy initialisation must not happen under capture), on a copy of the
         # first batch row only, so constructing the graph leaves slot / mass / position as they were.
-        if warmup > 0:
+        if warmup > 0 and n > 0:
             one = slice(0, 1)
             scratch = (slot[one].clone(), mass[one].clone(), position_ids[one].clone())
             side = torch.cuda.Stream(device=w_addr.device)
             side.wait_stream(torch.cuda.current_stream(w_addr.device))
             with torch.cuda.stream(side):
-                for j in range(min(warmup, n)):
-                    step(j, one, scratch)
+                steps(one, scratch)
             torch.cuda.current_stream(w_addr.device).wait_stream(side)
             del scratch
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph):  # records the launches; nothing runs until replay()
-            self.outputs = [step(j) for j in range(n)]
+            self.outputs = list(steps().unbind(0)) if n > 0 else []
 
     def replay(self) -> List[torch.Tensor]:
         """Run the ``n`` captured steps on the current contents of the static buffers."""
