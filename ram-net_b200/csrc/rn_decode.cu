@@ -41,7 +41,7 @@ struct RnDecodeParams {
     float norm_eps;
     int B, H, U, P, C, E, A;
     // consecutive steps of one launch and the element strides between their inputs and outputs
-    int steps;
+    int steps, pos_add;  // pos_add: on top of the positions
     int64_t st_addr[2], st_x, st_gamma, st_gate, st_y;
     int K[2];
     float re_norm[2];
@@ -57,16 +57,14 @@ __device__ __forceinline__ int64_t rn_in_row(const RnDecodeParams &p, const int 
     return b * ld + int64_t(h) * per_head;
 }
 
-// Four warps move the rows, two more decode the write and the read address; with several steps the decoders are one step
-// ahead.  A warp requests four rows before it uses the first; gains and read coefficients are computed one per lane.
 template <typename T, int KPL, int PPL>
-__global__ void __launch_bounds__(RN_DEC_THREADS) rn_decode_kernel(const RnDecodeParams p) {
-    extern __shared__ float dyn[];  // xs[2][C] | yred[4][C]
+__global__ void __launch_bounds__(RN_DEC_WARPS * 32) rn_decode_kernel(const RnDecodeParams p) {
+    extern __shared__ float dyn[];  // xs[C] | yred[4][C]
     __shared__ RnPairTable tabs[2];
     __shared__ RnWarpScratch scratch[2];
     __shared__ int row_off[RN_KMAX + 1];
-    __shared__ int sel_slot[2][2][RN_KMAX];  // by parity of the step
-    __shared__ float sel_val[2][2][RN_KMAX];
+    __shared__ int sel_slot[2][RN_KMAX];
+    __shared__ float sel_val[2][RN_KMAX];
     __shared__ float red[RN_DEC_WARPS][2];
     __shared__ float bcast;
 
@@ -74,65 +72,233 @@ __global__ void __launch_bounds__(RN_DEC_THREADS) rn_decode_kernel(const RnDecod
     const int b = bh / p.H, h = bh % p.H;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int C = p.C;
+    T *y = static_cast<T *>(p.y) + int64_t(bh) * C;
 
     if (p.mask != nullptr && p.mask[b] == 0) {
-        for (int step = 0; step < p.steps; ++step) {
-            T *y = static_cast<T *>(p.y) + step * p.st_y + int64_t(bh) * C;
-            for (int c = tid; c < C; c += RN_DEC_THREADS) y[c] = rn_from_float<T>(0.f);
-        }
+        for (int c = tid; c < C; c += blockDim.x) y[c] = rn_from_float<T>(0.f);
         return;
     }
+
+    float *xs = dyn;
+    float *yred = dyn + C;
+
+    rn_build_pairs(&tabs[0], p.K[0], row_off);
+    if (p.K[1] != p.K[0]) rn_build_pairs(&tabs[1], p.K[1], row_off);
+    const RnPairTable *tab_r = (p.K[1] != p.K[0]) ? &tabs[1] : &tabs[0];
+
+    if (warp < 2) {
+        RnDigitLoader<T> load;
+        load.base = static_cast<const T *>(warp == 0 ? p.w_addr : p.r_addr) + rn_in_row(p, bh, p.ld_addr[warp == 0 ? 0 : 1], p.U * p.P);
+        load.su = p.P;
+        load.sp = 1;
+        const int K = p.K[warp];
+        const RnDecoded<KPL> d =
+            rn_warp_decode<KPL, PPL>(load, p.U, p.P, K, p.re_norm[warp], &scratch[warp], warp == 0 ? &tabs[0] : tab_r, lane);
+        const int shift = (h < p.E) ? rn_pos_mod(rn_pos_at(p.pos, b, 0) + p.pos_add, p.A) : 0;
+#pragma unroll
+        for (int r = 0; r < KPL; ++r) {
+            const int e = lane * KPL + r;
+            if (e < K) {
+                sel_slot[warp][e] = rn_cape(d.idx[r], shift, p.A);
+                sel_val[warp][e] = d.val[r];
+            }
+        }
+    } else {
+        const T *x = static_cast<const T *>(p.x) + rn_in_row(p, bh, p.ld_x, C);
+        for (int c = tid - 64; c < C; c += 64) xs[c] = rn_to_float<T>(x[c]);
+    }
+    for (int c = tid; c < RN_DEC_WARPS * C; c += blockDim.x) yred[c] = 0.f;
+    __syncthreads();
+
+    const float gamma = rn_to_float<T>(static_cast<const T *>(p.gamma)[rn_in_row(p, bh, p.ld_gamma, 1)]);
+    float *slot = p.slot + int64_t(bh) * p.A * C;
+    float *mass = p.mass + int64_t(bh) * p.A;
+    const bool vec4 = (C & 3) == 0;
+
+    // ---- write: gated update of the selected rows ---------------------------------------------
+    for (int k = warp; k < p.K[0]; k += RN_DEC_WARPS) {
+        const float w = sel_val[0][k];
+        if (w == 0.f) continue;
+        const int a = sel_slot[0][k];
+        const RnGate g = rn_gate(w, gamma, mass[a], p.eps);
+        float *row = slot + int64_t(a) * C;
+        if (vec4) {
+            for (int c = lane * 4; c < C; c += 128) {
+                float4 s = *reinterpret_cast<float4 *>(row + c);
+                const float4 xv = *reinterpret_cast<const float4 *>(xs + c);
+                s.x = fmaf(g.gain, xv.x - s.x, s.x);
+                s.y = fmaf(g.gain, xv.y - s.y, s.y);
+                s.z = fmaf(g.gain, xv.z - s.z, s.z);
+                s.w = fmaf(g.gain, xv.w - s.w, s.w);
+                *reinterpret_cast<float4 *>(row + c) = s;
+            }
+        } else {
+            for (int c = lane; c < C; c += 32) row[c] = fmaf(g.gain, xs[c] - row[c], row[c]);
+        }
+        __syncwarp();
+        if (lane == 0) mass[a] = g.mass;
+    }
+    __syncthreads();
+
+    // ---- read: weighted sum of the selected rows (after this step's writes) --------------------
+    float sum_r = 0.f, sum_rm = 0.f;
+    float *acc = yred + warp * C;
+    for (int k = warp; k < p.K[1]; k += RN_DEC_WARPS) {
+        const float r = sel_val[1][k];
+        if (r == 0.f) continue;
+        const int a = sel_slot[1][k];
+        float coef = r;
+        if (p.mass_aware) {
+            coef = r * mass[a];
+            sum_r += r;
+            sum_rm += coef;
+        }
+        const float *row = slot + int64_t(a) * C;
+        if (vec4) {
+            for (int c = lane * 4; c < C; c += 128) {
+                const float4 s = *reinterpret_cast<const float4 *>(row + c);
+                float4 o = *reinterpret_cast<float4 *>(acc + c);
+                o.x = fmaf(coef, s.x, o.x);
+                o.y = fmaf(coef, s.y, o.y);
+                o.z = fmaf(coef, s.z, o.z);
+                o.w = fmaf(coef, s.w, o.w);
+                *reinterpret_cast<float4 *>(acc + c) = o;
+            }
+        } else {
+            for (int c = lane; c < C; c += 32) acc[c] = fmaf(coef, row[c], acc[c]);
+        }
+    }
+    if (lane == 0) {
+        red[warp][0] = sum_r;
+        red[warp][1] = sum_rm;
+    }
+    __syncthreads();
+
+    float scale = 1.f;
+    if (p.mass_aware) {
+        float sr = 0.f, srm = 0.f;
+        for (int w = 0; w < RN_DEC_WARPS; ++w) {
+            sr += red[w][0];
+            srm += red[w][1];
+        }
+        scale = sr / (srm + p.eps);
+    }
+    const bool epilogue = p.norm_weight != nullptr || p.gate != nullptr;
+    float sq = 0.f;
+    for (int c = tid; c < C; c += blockDim.x) {
+        float v = 0.f;
+        for (int w = 0; w < RN_DEC_WARPS; ++w) v += yred[w * C + c];
+        v *= scale;
+        if (epilogue) {
+            yred[c] = v;  // column c is owned by this thread in every pass
+            sq += v * v;
+        } else {
+            y[c] = rn_from_float<T>(v);
+        }
+    }
+    if (!epilogue) return;
+
+    float inv_rms = 1.f;
+    if (p.norm_weight != nullptr) {
+        sq = rn_warp_sum(sq);
+        __syncthreads();  // red[] is reused
+        if (lane == 0) red[warp][0] = sq;
+        __syncthreads();
+        if (tid == 0) {
+            float s = 0.f;
+            for (int w = 0; w < RN_DEC_WARPS; ++w) s += red[w][0];
+            bcast = rsqrtf(s / float(C) + p.norm_eps);
+        }
+        __syncthreads();
+        inv_rms = bcast;
+    }
+    const T *gate = p.gate ? static_cast<const T *>(p.gate) + rn_in_row(p, bh, p.ld_gate, C) : nullptr;
+    for (int c = tid; c < C; c += blockDim.x) {
+        float v = yred[c];
+        if (p.norm_weight != nullptr) v = v * inv_rms * p.norm_weight[c];
+        if (gate != nullptr) v = v / (1.f + expf(-rn_to_float<T>(gate[c])));
+        y[c] = rn_from_float<T>(v);
+    }
+}
+
+// The same with the shorter chain of latencies, for as many pairs as have a CTA at once: two more warps decode, one turn
+// (pair, step) ahead of the four that move rows, and a warp requests four rows before it uses the first (gains and read
+// coefficients are computed one per lane).  It has four CTAs of 192 threads an SM
+// where the kernel above has seven of 128 and fewer instructions: with more pairs the kernel above is faster.
+template <typename T, int KPL, int PPL>
+__global__ void __launch_bounds__(RN_DEC_THREADS, KPL == 1 ? 4 : 3) rn_decode_ahead_kernel(const RnDecodeParams p) {
+    extern __shared__ float dyn[];  // xs[2][C] | yred[4][C]
+    __shared__ RnPairTable tabs[2];
+    __shared__ RnWarpScratch scratch[2];
+    __shared__ int row_off[RN_KMAX + 1];
+    __shared__ int sel_slot[2][2][RN_KMAX];  // by parity of the turn
+    __shared__ float sel_val[2][2][RN_KMAX];
+    __shared__ float red[RN_DEC_WARPS][2];
+    __shared__ float bcast;
+
+    const int BH = p.B * p.H;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int C = p.C;
 
     float *yred = dyn + 2 * C;
 
     rn_build_pairs(&tabs[0], p.K[0], row_off);
     if (p.K[1] != p.K[0]) rn_build_pairs(&tabs[1], p.K[1], row_off);
 
+    int par = 0;
     if (warp >= RN_DEC_WARPS) {
-        // ================================ decoders ==========================================================
+        // ================================ addresses =========================================================
         const int which = warp - RN_DEC_WARPS, K = p.K[which];
-        const RnPairTable *tab = &tabs[p.K[1] != p.K[0] ? which : 0];
-        const int pos = h < p.E ? rn_pos_at(p.pos, b, 0) : 0;
-        const T *src = static_cast<const T *>(which ? p.r_addr : p.w_addr) + rn_in_row(p, bh, p.ld_addr[which], p.U * p.P);
 #pragma unroll 1
-        for (int step = 0; step < p.steps; ++step) {
+        for (int bh = blockIdx.x, step = 0; bh < BH; step + 1 < p.steps ? ++step : (step = 0, bh += gridDim.x)) {
+            const int b = bh / p.H, h = bh - b * p.H;
+            if (p.mask != nullptr && p.mask[b] == 0) continue;
             RnDigitLoader<T> load;
-            load.base = src + step * p.st_addr[which];
+            load.base = static_cast<const T *>(which ? p.r_addr : p.w_addr) + rn_in_row(p, bh, p.ld_addr[which], p.U * p.P) + step * p.st_addr[which];
             load.su = p.P;
             load.sp = 1;
-            const RnDecoded<KPL> d = rn_warp_decode<KPL, PPL>(load, p.U, p.P, K, p.re_norm[which], &scratch[which], tab, lane);
-            const int shift = (h < p.E) ? rn_pos_mod(pos + step, p.A) : 0;
+            const RnDecoded<KPL> d =
+                rn_warp_decode<KPL, PPL>(load, p.U, p.P, K, p.re_norm[which], &scratch[which], &tabs[p.K[1] != p.K[0] ? which : 0], lane);
+            const int shift = (h < p.E) ? rn_pos_mod(rn_pos_at(p.pos, b, 0) + step, p.A) : 0;
 #pragma unroll
             for (int r = 0; r < KPL; ++r) {
                 const int e = lane * KPL + r;
                 if (e < K) {
-                    sel_slot[step & 1][which][e] = rn_cape(d.idx[r], shift, p.A);
-                    sel_val[step & 1][which][e] = d.val[r];
+                    sel_slot[par][which][e] = rn_cape(d.idx[r], shift, p.A);
+                    sel_val[par][which][e] = d.val[r];
                 }
             }
-            __syncthreads();  // the step's addresses are there, those of the step before have been used
+            par ^= 1;
+            __syncthreads();  // the addresses are there, those of the turn before have been used
         }
         return;
     }
 
     // ================================ rows ==================================================================
-    // the decoders have left once the last step's addresses are there: what follows are barriers of these four warps
+    // the decoders leave once the last addresses are there: what follows are barriers of these four warps
     auto rows_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(RN_DEC_WARPS * 32) : "memory"); };
-    float *slot = p.slot + int64_t(bh) * p.A * C;
-    float *mass = p.mass + int64_t(bh) * p.A;
     const bool vec4 = (C & 3) == 0, epilogue = p.norm_weight != nullptr || p.gate != nullptr;
+    // one turn per pair and step
 #pragma unroll 1
-    for (int step = 0; step < p.steps; ++step) {
-        float *xs = dyn + (step & 1) * C;
+    for (int bh = blockIdx.x, step = 0; bh < BH; step + 1 < p.steps ? ++step : (step = 0, bh += gridDim.x)) {
+        const int b = bh / p.H;
+        float *slot = p.slot + int64_t(bh) * p.A * C;
+        float *mass = p.mass + int64_t(bh) * p.A;
+        float *xs = dyn + par * C;
         T *y = static_cast<T *>(p.y) + step * p.st_y + int64_t(bh) * C;
+        if (p.mask != nullptr && p.mask[b] == 0) {
+            for (int c = tid; c < C; c += RN_DEC_WARPS * 32) y[c] = rn_from_float<T>(0.f);
+            continue;
+        }
         {
             const T *x = static_cast<const T *>(p.x) + step * p.st_x + rn_in_row(p, bh, p.ld_x, C);
             for (int c = tid; c < C; c += RN_DEC_WARPS * 32) xs[c] = rn_to_float<T>(x[c]);
         }
         const float gamma = rn_to_float<T>(static_cast<const T *>(p.gamma)[step * p.st_gamma + rn_in_row(p, bh, p.ld_gamma, 1)]);
         __syncthreads();
-        const int *ws = sel_slot[step & 1][0], *rs = sel_slot[step & 1][1];
-        const float *wv = sel_val[step & 1][0], *rv = sel_val[step & 1][1];
+        const int *ws = sel_slot[par][0], *rs = sel_slot[par][1];
+        const float *wv = sel_val[par][0], *rv = sel_val[par][1];
+        par ^= 1;
 
         // ---- write: gated update of the selected rows; lane i of a group of four rows has the gain of row i ---------
         if (vec4) {
@@ -296,7 +462,7 @@ __global__ void __launch_bounds__(RN_DEC_THREADS) rn_decode_kernel(const RnDecod
                 y[c] = rn_from_float<T>(v);
             }
         }
-        // the barrier at the head of the next step keeps what this one still reads (yred, red) from being written to
+        // the barrier at the head of the next turn keeps what this one still reads (yred, red) from being written to
     }
 }
 
@@ -1130,7 +1296,7 @@ static int rn_launch_decode_fast_c(const RnDecodeParams &p, cudaStream_t stream)
 
 // 0 = launched, -1 = no specialised kernel for this shape
 template <typename T>
-static int rn_launch_decode_fast(const RnDecodeParams &p, int device, cudaStream_t stream) {
+static int rn_launch_decode_special(const RnDecodeParams &p, bool ahead, int device, cudaStream_t stream) {
     if (p.K[0] != p.K[1]) return -1;
     const size_t esz = sizeof(T);
     const uintptr_t io = reinterpret_cast<uintptr_t>(p.w_addr) | reinterpret_cast<uintptr_t>(p.r_addr) |
@@ -1139,6 +1305,7 @@ static int rn_launch_decode_fast(const RnDecodeParams &p, int device, cudaStream
     if ((io & 15) != 0 || (size_t(p.U) * p.P * esz) % 16 != 0) return -1;
     if (((p.ld_addr[0] | p.ld_addr[1] | p.ld_x | p.ld_gate | p.st_addr[0] | p.st_addr[1] | p.st_x | p.st_gate) * int64_t(esz)) % 16 != 0) return -1;
     if (rn_launch_decode_pair<T>(p, device, stream) == 0) return 0;
+    if (ahead) return -1;
     if (p.U == 2 && p.P == 64 && p.K[0] == 16) return rn_launch_decode_fast_c<T, 2, 64, 16>(p, stream);
     if (p.U == 3 && p.P == 32 && p.K[0] == 8) return rn_launch_decode_fast_c<T, 3, 32, 8>(p, stream);
     if (p.U == 2 && p.P == 16 && p.K[0] == 4) return rn_launch_decode_fast_c<T, 2, 16, 4>(p, stream);
@@ -1147,18 +1314,46 @@ static int rn_launch_decode_fast(const RnDecodeParams &p, int device, cudaStream
 
 static int rn_per_lane_dec(int64_t n) { return n <= 32 ? 1 : (n <= 64 ? 2 : 4); }
 
-template <typename T>
-static int rn_launch_decode(const RnDecodeParams &p, int kpl, int ppl, int grid, size_t smem, cudaStream_t stream) {
-#define RN_CASE(KP, PP)                                                                       \
-    if (kpl == KP && ppl == PP) {                                                             \
-        rn_decode_kernel<T, KP, PP><<<grid, RN_DEC_THREADS, smem, stream>>>(p);            \
-        return 0;                                                                             \
+// AHEAD: rn_decode_ahead_kernel, else one launch of rn_decode_kernel for every step
+template <typename T, bool AHEAD>
+static int rn_launch_decode(RnDecodeParams p, int kpl, int ppl, cudaStream_t stream) {
+    const int pairs = p.B * p.H, steps = p.steps;
+    const size_t smem = size_t(p.C) * (AHEAD ? 2 + RN_DEC_WARPS : 1 + RN_DEC_WARPS) * sizeof(float);
+#define RN_CASE(KP, PP)                                                                                              \
+    if (kpl == KP && ppl == PP) {                                                                                    \
+        if (AHEAD) {                                                                                                 \
+            rn_decode_ahead_kernel<T, KP, PP><<<pairs, RN_DEC_THREADS, smem, stream>>>(p);                           \
+            return 0;                                                                                                \
+        }                                                                                                            \
+        for (int s = 0; s < steps; ++s) {                                                                            \
+            rn_decode_kernel<T, KP, PP><<<pairs, RN_DEC_WARPS * 32, smem, stream>>>(p);                              \
+            p.w_addr = static_cast<const T *>(p.w_addr) + p.st_addr[0];                                              \
+            p.r_addr = static_cast<const T *>(p.r_addr) + p.st_addr[1];                                              \
+            p.x = static_cast<const T *>(p.x) + p.st_x;                                                              \
+            p.gamma = static_cast<const T *>(p.gamma) + p.st_gamma;                                                  \
+            if (p.gate) p.gate = static_cast<const T *>(p.gate) + p.st_gate;                                         \
+            p.y = static_cast<T *>(p.y) + p.st_y;                                                                    \
+            ++p.pos_add;                                                                                             \
+        }                                                                                                            \
+        return 0;                                                                                                    \
     }
     RN_CASE(1, 1) RN_CASE(1, 2) RN_CASE(1, 4) RN_CASE(2, 1) RN_CASE(2, 2) RN_CASE(2, 4) RN_CASE(4, 1) RN_CASE(4, 2)
     RN_CASE(4, 4)
 #undef RN_CASE
     rn_set_error("no decode kernel for K-per-lane=%d, P-per-lane=%d", kpl, ppl);
     return 1;
+}
+
+template <typename T>
+static int rn_launch_decode_step(const RnDecodeParams &p, int device, cudaStream_t stream) {
+    // As long as every pair has a CTA at once, the general kernel with the decoders ahead beats those of this file that take
+    // 16 pairs per CTA: for several steps (16 steps of 256 pairs, U2 P64 K16 f32: 314 -> 98 us; U2 P16 K4: 109 -> 54) and for a
+    // single one from 16 rows on (17.8 -> 10.4 us; with 4 rows 6.9 against 7.3).
+    const int K = p.K[0] > p.K[1] ? p.K[0] : p.K[1], kpl = rn_per_lane_dec(K), ppl = rn_per_lane_dec(p.P);
+    const bool ahead = p.B * p.H <= (kpl == 1 ? 4 : 3) * rn_sm_count(device) && (p.steps > 1 || K >= 16);
+    const int rc = rn_launch_decode_special<T>(p, ahead, device, stream);
+    if (rc >= 0) return rc;
+    return ahead ? rn_launch_decode<T, true>(p, kpl, ppl, stream) : rn_launch_decode<T, false>(p, kpl, ppl, stream);
 }
 
 // 1 when rn_decode_step_scaled() takes logit scales for this shape (the one-warp-per-pair kernel does), else 0
@@ -1259,23 +1454,11 @@ extern "C" int rn_decode_steps(const void *w_addr, const void *r_addr, const voi
     p.status = rn_status_word(device);
     RN_REQUIRE(p.status != nullptr, "cannot locate the status word of device %d", device);
 
-    const int kpl = rn_per_lane_dec(Kw > Kr ? Kw : Kr), ppl = rn_per_lane_dec(P);
-    const size_t smem = size_t(C) * (2 + RN_DEC_WARPS) * sizeof(float);
-    const int grid = int(B * H);
-    int rc;
     rn_prof_reset();
     rn_prof_mark(cudaStream_t(stream));
-    rc = dtype == RN_F32 ? rn_launch_decode_fast<float>(p, device, cudaStream_t(stream))
-         : dtype == RN_F16 ? rn_launch_decode_fast<__half>(p, device, cudaStream_t(stream))
-                           : rn_launch_decode_fast<__nv_bfloat16>(p, device, cudaStream_t(stream));
-    if (rc == 0) {
-        RN_CUDA(cudaGetLastError());
-        rn_prof_mark(cudaStream_t(stream));
-        return 0;
-    }
-    if (dtype == RN_F32) rc = rn_launch_decode<float>(p, kpl, ppl, grid, smem, cudaStream_t(stream));
-    else if (dtype == RN_F16) rc = rn_launch_decode<__half>(p, kpl, ppl, grid, smem, cudaStream_t(stream));
-    else rc = rn_launch_decode<__nv_bfloat16>(p, kpl, ppl, grid, smem, cudaStream_t(stream));
+    const int rc = dtype == RN_F32   ? rn_launch_decode_step<float>(p, device, cudaStream_t(stream))
+                   : dtype == RN_F16 ? rn_launch_decode_step<__half>(p, device, cudaStream_t(stream))
+                                     : rn_launch_decode_step<__nv_bfloat16>(p, device, cudaStream_t(stream));
     if (rc) return rc;
     RN_CUDA(cudaGetLastError());
     rn_prof_mark(cudaStream_t(stream));
