@@ -74,17 +74,27 @@ template <bool CLUSTER>
 __device__ __forceinline__ bool rn_mbar_wait(uint32_t bar, uint32_t parity) {  // bounded: about a second
     return rn_mbar_try<CLUSTER>(bar, parity) || rn_mbar_wait_slow<CLUSTER>(bar, parity);
 }
-// barrier of the compute warps; the answer is whether any of their threads brought `bad`
-__device__ __forceinline__ bool rn_compute_sync(bool bad) {
+// barrier ID of THREADS threads; the answer is whether any of them brought `bad`
+template <int ID, int THREADS>
+__device__ __forceinline__ bool rn_bar_or(bool bad) {
     uint32_t any;
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-                 : "=r"(any) : "r"(uint32_t(bad)), "n"(RN_AP_COMPUTE) : "memory");
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, %2, %3, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(any) : "r"(uint32_t(bad)), "n"(ID), "n"(THREADS) : "memory");
     return any != 0;
 }
+__device__ __forceinline__ bool rn_compute_sync(bool bad) { return rn_bar_or<1, RN_AP_COMPUTE>(bad); }
+__device__ __forceinline__ float rn_dot4(float4 a, float4 b) { return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, a.w * b.w))); }
+// the same whichever half a unit holds first: which unit has a row varies from run to run
+__device__ __forceinline__ float rn_dot8(float4 a0, float4 b0, float4 a1, float4 b1) { return rn_dot4(a0, b0) + rn_dot4(a1, b1); }
+__device__ __forceinline__ void rn_stg_f4(float *p, float4 v) { __stcs(reinterpret_cast<float4 *>(p), v); }
 
-template <typename T, int CS>
+// MODE: RN_FORWARD, or RN_REPLAY, the first sweep of the backward pass, over lists of its own (rn_bwd_lists.cu): it runs the state
+// again, the gather takes <row, d_y> of every read instead of sums (no y, hence no cluster), the update stores x - row of every
+// write for the reverse sweep.  The reads of an owner are dealt evenly to the units, since nothing is summed over a token.
+template <typename T, int CS, int MODE>
 __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnListParams p) {
     constexpr int LPU = CS / 4;                    // lanes of a row (state and x transfers, y)
+    constexpr bool Y = MODE != RN_REPLAY;          // rows of y (d_x) are finished
     constexpr int ROW = CS * 4;                    // bytes of a row
     constexpr int XT = RN_LST_LMAX * LPU / RN_AP_SERVICE;  // x pieces per service thread
     extern __shared__ __align__(128) unsigned char dyn[];
@@ -104,8 +114,8 @@ __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnList
 
     unsigned char *S = dyn;                        // [rows][CS] f32
     unsigned char *xt = S + (size_t(ROW) << p.lr); // [2][L][CS]; read entries count its rows on from those of S
-    unsigned char *yb = xt + size_t(2 * L) * ROW;  // [2][N sources][Lq][CS] (N > 1)
-    unsigned char *lists = yb + (N > 1 ? size_t(2 * L) * ROW : 0);
+    unsigned char *yb = xt + size_t(2 * L) * ROW;  // [2][N sources][Lq][CS] (N > 1); RN_REPLAY: d_y, as xt
+    unsigned char *lists = yb + (N > 1 || !Y ? size_t(2 * L) * ROW : 0);
     const uint32_t bar0 = rn_smem_u32(bars);
     auto FULL = [&](int s) { return bar0 + (s & 1) * 8u; };
     auto FREE = [&](int s) { return bar0 + 16u + (s & 1) * 8u; };
@@ -131,7 +141,7 @@ __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnList
     const int words = rn_touch_words(p.lr);
     const uint32_t *touch = p.touch ? p.touch + ((int64_t(bh) << lg) + own) * 2 * words : nullptr;
     __syncthreads();
-    if (N > 1) rn_cluster_sync();  // every CTA's barriers are set up before the first remote arrival
+    if (Y && N > 1) rn_cluster_sync();  // every CTA's barriers are set up before the first remote arrival
 
     bool failed = false;
     if (tid >= RN_AP_COMPUTE) {
@@ -146,14 +156,30 @@ __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnList
         uint32_t peer_free = 0;
         if (sid < N) peer_free = rn_mapa(bar0 + 48u, uint32_t(sid));
 
-        // x of the step that comes next: requested a step ahead, kept as loaded until it is put into shared memory
-        RnRaw4<T> xr[XT];
+        // x of the block that comes next: requested a block ahead, kept as loaded until it is put into shared memory
+        RnRaw4<T> xr[XT], dr[Y ? 1 : XT];
+        const T *dy = Y ? nullptr : static_cast<const T *>(p.dy) + b * p.dyb + h * p.dyh + ch;
         int ptok[2] = {0, 0}, plen[2] = {0, 0};            // tokens of the two steps before, by parity
-        const int64_t xstep = int64_t(TSTEP) * p.xt;
-        // The table is read two steps ahead, x one; the copy of a list starts as soon as its buffer is free.  Turn -1 only
+        auto request = [&](int bk) {
+            const int len = chan_ok ? p.T - bk * L - st0 : 0;
+            const T *src = x + int64_t(bk * L + st0) * p.xt, *dsrc = Y ? nullptr : dy + int64_t(bk * L + st0) * p.dyt;
+#pragma unroll
+            for (int i = 0; i < XT; ++i) {
+                xr[i] = rn_zero_raw4<T>();
+                if (i * TSTEP < len && st0 + i * TSTEP < L) xr[i] = rn_load_raw4<T>(src);
+                src += int64_t(TSTEP) * p.xt;
+                if constexpr (!Y) {
+                    dr[i] = rn_zero_raw4<T>();
+                    if (i * TSTEP < len && st0 + i * TSTEP < L) dr[i] = rn_load_raw4<T>(dsrc);
+                    dsrc += int64_t(TSTEP) * p.dyt;
+                }
+            }
+        };
+        // The table is read two steps ahead, x a block; the copy of a list starts as soon as its buffer is free.  Turn -1 only
         // requests the first x, the last two turns only finish y: every part of the loop stands here once, which keeps
-        // the kernel's code small (instruction fetch is what a longer one would wait for)
-        int blk = 0, st = 0, cur_blk = 0;
+        // the kernel's code small (instruction fetch is what a longer one would wait for).  Failure is collective: one warp
+        // that gives up takes the others along at the barrier of the turn.
+        int blk = 0, st = 0, cur_blk = -1, cur_st = 0;
         uint4 cur = make_uint4(0, 0, 0, 0), nxt = rn_step_entry(p, first, recs, 0, 0, own);
         int last = 1 << 30;
 #pragma unroll 1
@@ -163,44 +189,43 @@ __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnList
             uint4 nn = make_uint4(0, 0, 0, 0);
             if (rn_steps_of(nxt) != 0) nn = rn_step_entry(p, first, recs, nblk, nst, own);
             if (step >= 0 && step < last) {
-                const int cblk = cur_blk;
                 if (step >= 2 && !rn_mbar_wait<false>(FREE(step), phase(step - 2))) failed = true;
-                if (__any_sync(RN_FULL, failed || stop)) { failed = true; break; }
                 if (sid == 0) {
                     const uint32_t bytes = (cur.x >> 16) << 4;
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(FULL(step)), "r"(bytes) : "memory");
-                    rn_bulk_g2s(lists + size_t(step & 1) * p.list_max, recs + cblk * p.blk_bytes + data_at + (size_t(cur.x & 0xffffu) << 4), bytes,
-                                &bars[step & 1]);
+                    rn_bulk_g2s(lists + size_t(step & 1) * p.list_max, recs + cur_blk * p.blk_bytes + data_at + (size_t(cur.x & 0xffffu) << 4),
+                                bytes, &bars[step & 1]);
                 }
-                unsigned char *xd = xt + (size_t(step & 1) * L + st0) * ROW + ul * 16;
+                if (cur_st == 0) {
+                    const size_t at = (size_t(cur_blk & 1) * L + st0) * ROW + ul * 16;
 #pragma unroll
-                for (int i = 0; i < XT; ++i) rn_pin(xr[i]);
+                    for (int i = 0; i < XT; ++i) {
+                        rn_pin(xr[i]);
+                        if constexpr (!Y) rn_pin(dr[i]);
+                    }
 #pragma unroll
-                for (int i = 0; i < XT; ++i)
-                    if (st0 + i * TSTEP < L) *reinterpret_cast<float4 *>(xd + i * TSTEP * ROW) = rn_cvt_raw4(xr[i]);
+                    for (int i = 0; i < XT; ++i)
+                        if (st0 + i * TSTEP < L) {
+                            *reinterpret_cast<float4 *>(xt + at + i * TSTEP * ROW) = rn_cvt_raw4(xr[i]);
+                            if constexpr (!Y) *reinterpret_cast<float4 *>(yb + at + i * TSTEP * ROW) = rn_cvt_raw4(dr[i]);
+                        }
+                }
                 __syncwarp();
                 if (lane == 0) rn_mbar_arrive(FULL(step));
             }
-            if (rn_steps_of(nxt) != 0) {
-                const int len = chan_ok ? int(nxt.y >> 16) - st0 : 0;
-                const T *src = x + int64_t(blk * L + int(nxt.y & 0xffffu) + st0) * p.xt;
-#pragma unroll
-                for (int i = 0; i < XT; ++i) {
-                    xr[i] = rn_zero_raw4<T>();
-                    if (i * TSTEP < len) xr[i] = rn_load_raw4<T>(src);
-                    src += xstep;
-                }
-            } else if (step + 1 < last) {
-                last = step + 1;
+            if (step < last && cur_st == 0) {
+                if (cur_blk + 1 < p.nblocks) request(cur_blk + 1);
             }
-            if (N > 1) {
+            if (rn_steps_of(nxt) == 0 && step + 1 < last) last = step + 1;
+            if (Y && N > 1) {
+                bool arrive = false;
                 if (step >= 2) {                           // y of the step before the last, from the parts of all owners
                     const int s = step - 2, mine = max(0, min(Lq, plen[s & 1] - own * Lq));
-                    if (!rn_mbar_wait<true>(YFULL(s), phase(s))) { failed = true; break; }
+                    if (!rn_mbar_wait<true>(YFULL(s), phase(s))) failed = true;
                     const unsigned char *src = yb + (size_t(s & 1) * L + st0) * ROW + ul * 16;
                     T *dst = y + int64_t(ptok[s & 1] + own * Lq + st0) * p.yt;
 #pragma unroll 1
-                    for (int t = st0; t < mine; t += TSTEP) {
+                    for (int t = st0; t < mine && !failed; t += TSTEP) {
                         float4 a = *reinterpret_cast<const float4 *>(src);
 #pragma unroll 1
                         for (int o = 1; o < N; ++o) {
@@ -211,19 +236,23 @@ __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnList
                         src += TSTEP * ROW;
                         dst += int64_t(TSTEP) * p.yt;
                     }
-                    // all service warps are done with the buffer before the cluster hears of it
-                    asm volatile("barrier.cta.sync 2, %0;" ::"n"(RN_AP_SERVICE) : "memory");
-                    if (sid < N) rn_mbar_arrive_remote(peer_free + (s & 1) * 8u);
+                    arrive = true;
                 }
+                // all service warps are done with the buffer before the cluster hears of it
+                failed = rn_bar_or<2, RN_AP_SERVICE>(failed || stop);
+                if (failed) break;
+                if (arrive && sid < N) rn_mbar_arrive_remote(peer_free + (step & 1) * 8u);
                 if (step >= 0 && step < last) {
                     ptok[step & 1] = cur_blk * L + int(cur.y & 0xffffu);
                     plen[step & 1] = int(cur.y >> 16);
                 }
-            } else if (step >= last) {
-                break;
+            } else {
+                failed = rn_bar_or<2, RN_AP_SERVICE>(failed || stop);
+                if (failed || step >= last) break;
             }
             cur = nxt;
             cur_blk = blk;
+            cur_st = st;
             nxt = nn;
             blk = nblk;
             st = nst;
@@ -241,6 +270,12 @@ __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnList
         const uint32_t sl = rn_smem_u32(S) + lane_off, xl = rn_smem_u32(xt) + lane_off, yl = rn_smem_u32(yb) + uint32_t(own * Lq * ROW) + lane_off;
         const int ch0 = grp * CS + int(lane_off) / 4, ch1 = grp * CS + int(lane_off ^ HALF) / 4;
         T *y = static_cast<T *>(p.y) + b * p.yb + h * p.yh;
+        const uint32_t dy_tile = rn_smem_u32(yb) + lane_off;                                             // RN_REPLAY
+        // RN_REPLAY: this lane's channels of token 0, write 0 in the workspace of the reverse sweep, in slices of its width
+        auto delta_at = [&](int ch) {
+            return MODE == RN_REPLAY ? p.delta + (int64_t(bh) * ((C + p.dcs - 1) / p.dcs) + ch / p.dcs) * p.T * p.Kw * p.dcs + ch % p.dcs : nullptr;
+        };
+        float *const delta0 = delta_at(ch0), *const delta1 = delta_at(ch1);
         const int lq = 31 - __clz(Lq);
         {   // the rows into shared memory, eight requests of a thread at a time; the service warps fetch the first step meanwhile
             constexpr int LD = CS / 4, STEP = RN_AP_COMPUTE / LD;
@@ -272,16 +307,78 @@ __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnList
             const uint32_t tok = lst + 16, Wl = lst + (uint32_t(hd.atW) << 4);
             blk += t0 == 0;
 
-            // ---- gather: two entries at a time, the next two requested before they are used ---------------------------
-            float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            // ---- the units' shares ------------------------------------------------------------------------------------
+            const uint32_t tile = uint32_t(blk & 1) * uint32_t(L * ROW);
+            constexpr int LU = CS == 32 ? 7 : 8;               // log2 of NU
+            static_assert((1 << LU) == NU, "units");
+            [[maybe_unused]] auto share = [&](uint32_t table, uint32_t n, uint32_t &from, uint32_t &to) {  // run of unit u (rn_lists.cuh)
+                const uint32_t q = (n + NU - 1) >> LU;
+                from = to = n;
+                if (u * q < n) {
+                    from = rn_lds_u16(table + u * 2);
+                    if ((u + 1) * q < n && u + 1 < NU) to = rn_lds_u16(table + u * 2 + 2);
+                }
+            };
+            // ---- gather -------------------------------------------------------------------------------------------------
             int tk = -1;
-            if (tu < len) {
-                tk = rn_lds_u8(Wl - ((len + 15) & ~15) + tu);
+            float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if constexpr (MODE == RN_REPLAY) {
+                // <row, d_y> of every read: entries {coef, row of S or x | token << 12 | k << 19 | last of its read << 31} two at
+                // a time.  All units of a warp go round together (they shuffle); one that is through goes on with zeros.
+                float *out = p.part + ((int64_t(bh) * p.ngroups + grp) * p.T + blk * L) * p.Kr;
+                uint32_t q, end;
+                share(tok, hd.nR, q, end);
                 const uint32_t rl = lst + (uint32_t(hd.atR) << 4);
-                uint32_t q = rl + rn_lds_u16(tok + tk * 2) * 8u + part * 16u;
-                const uint32_t end = rl + rn_lds_u16(tok + tk * 2 + 2) * 8u;
+                q = rl + q * 8u;
+                end = rl + end * 8u;
+                const uint2 none = make_uint2(0, 0);
+                uint2 ea = none, eb = none;
+                if (q < end) ea = rn_lds_u2(q);
+                if (q + 8u < end) eb = rn_lds_u2(q + 8u);
+                uint32_t have = ~0u;                           // the token whose d_y is in d0, d1
+                float4 d0 = make_float4(0.f, 0.f, 0.f, 0.f), d1 = d0;
+                float run = 0.f;                               // per lane; summed over the lanes at the end of a read
+                auto dot = [&](uint32_t m, const float4 &r0, const float4 &r1) {
+                    const uint32_t t = m >> 12 & 0x7fu;
+                    if (t != have) {
+                        d0 = rn_lds_f4(dy_tile + tile + t * ROW);
+                        d1 = rn_lds_f4((dy_tile + tile + t * ROW) ^ HALF);
+                        have = t;
+                    }
+                    return rn_dot8(r0, d0, r1, d1);
+                };
+#pragma unroll 1
+                while (__any_sync(RN_FULL, q < end)) {
+                    const uint2 ca = ea, cb = eb;
+                    const uint32_t r0 = sl + (ca.y & 0xfffu) * ROW, r1 = sl + (cb.y & 0xfffu) * ROW;
+                    const float4 a0 = rn_lds_f4(r0), b0 = rn_lds_f4(r0 ^ HALF), a1 = rn_lds_f4(r1), b1 = rn_lds_f4(r1 ^ HALF);
+                    q += 16u;
+                    ea = eb = none;
+                    if (q < end) ea = rn_lds_u2(q);
+                    if (q + 8u < end) eb = rn_lds_u2(q + 8u);
+                    const float va = fmaf(__uint_as_float(ca.x), dot(ca.y, a0, b0), run);
+                    run = int(ca.y) < 0 ? 0.f : va;
+                    const float vb = fmaf(__uint_as_float(cb.x), dot(cb.y, a1, b1), run);
+                    run = int(cb.y) < 0 ? 0.f : vb;
+                    // even lanes add up the first entry, odd lanes the second
+                    float v = (ul & 1) ? vb : va;
+                    v += __shfl_xor_sync(RN_FULL, (ul & 1) ? va : vb, 1);
+#pragma unroll
+                    for (int o = 2; o < LPU; o <<= 1) v += __shfl_xor_sync(RN_FULL, v, o);
+                    const uint32_t m = (ul & 1) ? cb.y : ca.y;
+                    if (ul < 2 && int(m) < 0) out[int(m >> 12 & 0x7fu) * p.Kr + int(m >> 19 & 0x7fu)] = v;
+                }
+            } else {
+                // two entries at a time, the next two requested before they are used
+                uint32_t q = 0, end = 0;
                 uint4 e = make_uint4(0, 0, 0, 0);
-                if (q < end) e = rn_lds_u4(q);
+                if (tu < len) {
+                    tk = rn_lds_u8(Wl - ((len + 15) & ~15) + tu);
+                    const uint32_t rl = lst + (uint32_t(hd.atR) << 4);
+                    q = rl + rn_lds_u16(tok + tk * 2) * 8u + part * 16u;
+                    end = rl + rn_lds_u16(tok + tk * 2 + 2) * 8u;
+                    if (q < end) e = rn_lds_u4(q);
+                }
 #pragma unroll 1
                 while (q < end) {
                     const uint32_t r0 = sl + e.y, r1 = sl + e.w;
@@ -295,7 +392,7 @@ __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnList
                     acc[4] = fmaf(c1, b1.x, acc[4]); acc[5] = fmaf(c1, b1.y, acc[5]); acc[6] = fmaf(c1, b1.z, acc[6]); acc[7] = fmaf(c1, b1.w, acc[7]);
                 }
             }
-            if (upt > 1) {
+            if (Y && upt > 1) {
                 // units of a token take the halves in turns: first bring both to the even unit's order
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -310,12 +407,12 @@ __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnList
                 }
             }
             // the y buffers of this parity are free again in every CTA of the cluster
-            if (N > 1 && tid == 0 && step >= 2 && !rn_mbar_wait<true>(YFREE(step), phase(step - 2))) failed = true;
+            if (Y && N > 1 && tid == 0 && step >= 2 && !rn_mbar_wait<true>(YFREE(step), phase(step - 2))) failed = true;
             if (rn_compute_sync(failed || stop)) {
                 failed = true;
                 break;
             }
-            if (part == 0 && tk >= 0) {  // (an even unit where upt > 1)
+            if (Y && part == 0 && tk >= 0) {  // (an even unit where upt > 1)
                 if (N > 1) {  // to the CTA that finishes the token, at this owner's place
                     const uint32_t q = uint32_t(tk) >> lq;
                     const uint32_t at = rn_mapa(yl + (uint32_t(step & 1) * uint32_t(L) + (uint32_t(tk) & uint32_t(Lq - 1))) * ROW, q);
@@ -328,62 +425,73 @@ __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnList
                 }
             }
             // ---- update ------------------------------------------------------------------------------------------
-            {
-                const uint32_t xs = xl + uint32_t(step & 1) * uint32_t(L * ROW);
-                auto apply = [&](float4 &s, const float4 &xv, float g) {
-                    s.x = fmaf(g, xv.x - s.x, s.x);
-                    s.y = fmaf(g, xv.y - s.y, s.y);
-                    s.z = fmaf(g, xv.z - s.z, s.z);
-                    s.w = fmaf(g, xv.w - s.w, s.w);
-                };
-                // slots written more than once: the row stays in registers along the slot's writes
+            const uint32_t xs = xl + tile, starts = MODE == RN_REPLAY ? tok + min(int(hd.nR), NU) * 2 : tok + (len + 1) * 2;
+            const int64_t block_row = int64_t(blk * L) * p.Kw * p.dcs;
+            // x - row of a write, for the reverse sweep
+            auto keep = [&](uint32_t m, const float4 &s0, const float4 &s1, const float4 &x0, const float4 &x1) {
+                if constexpr (MODE == RN_REPLAY) {
+                    const int64_t at = block_row + (int(m >> 11 & 0x7fu) * p.Kw + int(m >> 18 & 0x7fu)) * p.dcs;
+                    if (ch0 < C) rn_stg_f4(delta0 + at, make_float4(x0.x - s0.x, x0.y - s0.y, x0.z - s0.z, x0.w - s0.w));
+                    if (ch1 < C) rn_stg_f4(delta1 + at, make_float4(x1.x - s1.x, x1.y - s1.y, x1.z - s1.z, x1.w - s1.w));
+                }
+            };
+            auto apply = [&](float4 &s, const float4 &xv, float g) {
+                s.x = fmaf(g, xv.x - s.x, s.x);
+                s.y = fmaf(g, xv.y - s.y, s.y);
+                s.z = fmaf(g, xv.z - s.z, s.z);
+                s.w = fmaf(g, xv.w - s.w, s.w);
+            };
+            // slots written more than once: the row stays in registers along the slot's writes
 #pragma unroll 1
-                for (int i = u; i < hd.nM; i += NU) {
-                    uint32_t q = Wl + rn_lds_u16(tok + (len + 1 + i) * 2) * 8u;
-                    uint2 e = rn_lds_u2(q), e1 = rn_lds_u2(q + 8u);
-                    const uint32_t cell = sl + (e.y & 0x7ffu) * ROW;
-                    float4 s0 = rn_lds_f4(cell), s1 = rn_lds_f4(cell ^ HALF);
-                    uint32_t xa = xs + ((e.y >> 11) & 0x7fu) * ROW;
-                    float4 x0 = rn_lds_f4(xa), x1 = rn_lds_f4(xa ^ HALF);
-                    for (;;) {  // the next write and its x are requested before this one is applied
-                        xa = xs + ((e1.y >> 11) & 0x7fu) * ROW;
-                        const float4 n0 = rn_lds_f4(xa), n1 = rn_lds_f4(xa ^ HALF);
-                        apply(s0, x0, __uint_as_float(e.x));
-                        apply(s1, x1, __uint_as_float(e.x));
-                        x0 = n0;
-                        x1 = n1;
-                        e = e1;
-                        if (int(e.y) < 0) break;
-                        q += 8u;
-                        e1 = rn_lds_u2(q + 8u);
-                    }
+            for (int i = u; i < hd.nM; i += NU) {
+                uint32_t q = Wl + rn_lds_u16(starts + i * 2) * 8u;
+                uint2 e = rn_lds_u2(q), e1 = rn_lds_u2(q + 8u);
+                const uint32_t cell = sl + (e.y & 0x7ffu) * ROW;
+                float4 s0 = rn_lds_f4(cell), s1 = rn_lds_f4(cell ^ HALF);
+                uint32_t xa = xs + ((e.y >> 11) & 0x7fu) * ROW;
+                float4 x0 = rn_lds_f4(xa), x1 = rn_lds_f4(xa ^ HALF);
+                for (;;) {  // the next write and its x are requested before this one is applied
+                    xa = xs + ((e1.y >> 11) & 0x7fu) * ROW;
+                    const float4 n0 = rn_lds_f4(xa), n1 = rn_lds_f4(xa ^ HALF);
+                    keep(e.y, s0, s1, x0, x1);
                     apply(s0, x0, __uint_as_float(e.x));
                     apply(s1, x1, __uint_as_float(e.x));
-                    rn_sts_f4(cell, s0);
-                    rn_sts_f4(cell ^ HALF, s1);
+                    x0 = n0;
+                    x1 = n1;
+                    e = e1;
+                    if (int(e.y) < 0) break;
+                    q += 8u;
+                    e1 = rn_lds_u2(q + 8u);
                 }
-                // slots written once
-                int i = u - (hd.nM & (NU - 1));  // units with a slot of the former kind more start behind the others
-                if (i < 0) i += NU;
-                uint2 e = make_uint2(0, 0);
-                if (i < hd.nS) e = rn_lds_u2(Wl + i * 8u);
+                keep(e.y, s0, s1, x0, x1);
+                apply(s0, x0, __uint_as_float(e.x));
+                apply(s1, x1, __uint_as_float(e.x));
+                rn_sts_f4(cell, s0);
+                rn_sts_f4(cell ^ HALF, s1);
+            }
+            // slots written once
+            int i = u - (hd.nM & (NU - 1));  // units with a slot of the former kind more start behind the others
+            if (i < 0) i += NU;
+            uint2 e = make_uint2(0, 0);
+            if (i < hd.nS) e = rn_lds_u2(Wl + i * 8u);
 #pragma unroll 1
-                while (i < hd.nS) {
-                    const uint32_t cell = sl + (e.y & 0x7ffu) * ROW, xa = xs + ((e.y >> 11) & 0x7fu) * ROW;
-                    const float g = __uint_as_float(e.x);
-                    float4 s0 = rn_lds_f4(cell), s1 = rn_lds_f4(cell ^ HALF);
-                    const float4 x0 = rn_lds_f4(xa), x1 = rn_lds_f4(xa ^ HALF);
-                    i += NU;
-                    if (i < hd.nS) e = rn_lds_u2(Wl + i * 8u);
-                    apply(s0, x0, g);
-                    apply(s1, x1, g);
-                    rn_sts_f4(cell, s0);
-                    rn_sts_f4(cell ^ HALF, s1);
-                }
+            while (i < hd.nS) {
+                const uint32_t cell = sl + (e.y & 0x7ffu) * ROW, xa = xs + ((e.y >> 11) & 0x7fu) * ROW;
+                const uint32_t m = e.y;
+                const float g = __uint_as_float(e.x);
+                float4 s0 = rn_lds_f4(cell), s1 = rn_lds_f4(cell ^ HALF);
+                const float4 x0 = rn_lds_f4(xa), x1 = rn_lds_f4(xa ^ HALF);
+                i += NU;
+                if (i < hd.nS) e = rn_lds_u2(Wl + i * 8u);
+                keep(m, s0, s1, x0, x1);
+                apply(s0, x0, g);
+                apply(s1, x1, g);
+                rn_sts_f4(cell, s0);
+                rn_sts_f4(cell ^ HALF, s1);
             }
             if (rn_compute_sync(false)) break;
             if (tid == 0) rn_mbar_arrive(FREE(step));
-            if (N > 1 && tid < N) rn_mbar_arrive_remote(rn_mapa(YFULL(step), uint32_t(tid)));
+            if (Y && N > 1 && tid < N) rn_mbar_arrive_remote(rn_mapa(YFULL(step), uint32_t(tid)));
             if ((hd.len & 0x8000) != 0) break;
         }
     }
@@ -392,7 +500,7 @@ __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnList
         atomicMax(p.status, RN_STATUS_WAIT_TIMEOUT);
     }
     __syncthreads();
-    if (!stop) {
+    if (!stop && p.slot_out != nullptr) {
         const int ul = tid % LPU, ch = grp * CS + ul * 4;
         float *dst = p.slot_out + int64_t(bh) * p.A * C + ch;
 #pragma unroll 1
@@ -402,12 +510,12 @@ __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnList
             if (on && ch < C && a < p.A) *reinterpret_cast<float4 *>(dst + int64_t(a) * C) = *reinterpret_cast<const float4 *>(S + size_t(r) * ROW + ul * 16);
         }
     }
-    if (N > 1) rn_cluster_sync();  // nobody's shared memory goes away while a store or arrival to it may be under way
+    if (Y && N > 1) rn_cluster_sync();  // nobody's shared memory goes away while a store or arrival to it may be under way
 }
 
-template <typename T, int CS>
+template <typename T, int CS, int MODE>
 static int rn_launch_apply_t(const RnListParams &p, const RnListPlan &pl, cudaStream_t stream) {
-    RN_CUDA(cudaFuncSetAttribute(rn_apply_kernel<T, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(pl.smem_apply)));
+    RN_CUDA(cudaFuncSetAttribute(rn_apply_kernel<T, CS, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(pl.smem_apply)));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(p.B) * unsigned(p.H) * unsigned(pl.ngroups) * unsigned(pl.N));
     cfg.blockDim = dim3(RN_AP_THREADS);
@@ -419,18 +527,27 @@ static int rn_launch_apply_t(const RnListParams &p, const RnListPlan &pl, cudaSt
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = pl.N > 1 ? 1 : 0;
-    RN_CUDA(cudaLaunchKernelEx(&cfg, rn_apply_kernel<T, CS>, p));
+    cfg.numAttrs = MODE != RN_REPLAY && pl.N > 1 ? 1 : 0;
+    RN_CUDA(cudaLaunchKernelEx(&cfg, rn_apply_kernel<T, CS, MODE>, p));
     return 0;
 }
 
 template <typename T>
-static int rn_launch_apply_cs(const RnListParams &p, const RnListPlan &pl, cudaStream_t stream) {
-    return pl.cs == 32 ? rn_launch_apply_t<T, 32>(p, pl, stream) : rn_launch_apply_t<T, 16>(p, pl, stream);
+static int rn_launch_mode(const RnListParams &p, const RnListPlan &pl, int mode, cudaStream_t stream) {
+    if (mode == RN_FORWARD) return pl.cs == 32 ? rn_launch_apply_t<T, 32, RN_FORWARD>(p, pl, stream) : rn_launch_apply_t<T, 16, RN_FORWARD>(p, pl, stream);
+    return pl.cs == 32 ? rn_launch_apply_t<T, 32, RN_REPLAY>(p, pl, stream) : rn_launch_apply_t<T, 16, RN_REPLAY>(p, pl, stream);
+}
+
+static int rn_launch_dtype(const RnListParams &p, const RnListPlan &pl, int mode, int dtype, cudaStream_t stream) {
+    if (dtype == RN_F32) return rn_launch_mode<float>(p, pl, mode, stream);
+    if (dtype == RN_F16) return rn_launch_mode<__half>(p, pl, mode, stream);
+    return rn_launch_mode<__nv_bfloat16>(p, pl, mode, stream);
 }
 
 int rn_launch_apply(const RnListParams &p, const RnListPlan &pl, int dtype, cudaStream_t stream) {
-    if (dtype == RN_F32) return rn_launch_apply_cs<float>(p, pl, stream);
-    if (dtype == RN_F16) return rn_launch_apply_cs<__half>(p, pl, stream);
-    return rn_launch_apply_cs<__nv_bfloat16>(p, pl, stream);
+    return rn_launch_dtype(p, pl, RN_FORWARD, dtype, stream);
+}
+
+int rn_launch_replay(const RnListParams &p, const RnListPlan &pl, int dtype, cudaStream_t stream) {
+    return rn_launch_dtype(p, pl, RN_REPLAY, dtype, stream);
 }

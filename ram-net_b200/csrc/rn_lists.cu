@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(RN_LISTS_THREADS, 1) rn_lists_kernel(const RnL
             if (cnt[j] == 0u) continue;
             const uint32_t o = ws[j] >> lr, q = (tab[ws[j]] >> 16) + rank[j];
             reinterpret_cast<uint2 *>(img + (at_W[o] << 4))[q] =
-                make_uint2(0u, (ws[j] & uint32_t(row_mask)) | (uint32_t(t - t0) << 11) | (uint32_t(part * kw + j) << 18) | (rank[j] + 1u == cnt[j] ? 1u << 31 : 0u));
+                make_uint2(0u, (ws[j] & uint32_t(row_mask)) | (uint32_t(t) << 11) | (rank[j] + 1u == cnt[j] ? 1u << 31 : 0u));
             // rn_alpha() with the exponential taken once per token
             const float cw = 1.f - wv[j];
             const float alpha = (gate >= 0.f ? cw * eg : cw) / (gate >= 0.f ? wv[j] + eg * cw : cw + eg * wv[j]);
@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(RN_GAINS_THREADS) rn_gains_kernel(const RnList
             *cell = m;
         }
         __syncthreads();
-        const uint32_t xrow = uint32_t(rows) + uint32_t(step & 1) * uint32_t(p.L);
+        const uint32_t xrow = uint32_t(rows) + uint32_t(blk & 1) * uint32_t(p.L);
         auto settle = [&](int i, float c, uint32_t m) {       // coefficients of a read
             const int n = int((m >> 22) & 0x1ffu), q = int((m >> 11) & 0x7ffu);
             float one = 0.f;

@@ -29,10 +29,10 @@
 //                                        zero);  u16 start[nM]  first write of
 //                                        every slot that is written more than once
 //                   u8 perm[len]         the tokens, those with most read entries first
-//                   {f32 gain, u32 row | token << 11 | k << 18 | last of its slot << 31}[nW]   the nS slots that are
+//                   {f32 gain, u32 row | token of the block << 11 | last of its slot << 31}[nW]   the nS slots that are
 //                                        written once, then the others, slot by slot in time order
 //                   {f32 coef, u32 ref}[nR]   ref: byte offset from the owner's first row, of a row of the state or of x
-//                                        (which follow them: x(token) of the step is row rows + parity * L + token)
+//                                        (which follow them: x(token of the block) is row rows + parity of the block * L + token)
 //                   -- up to here copied by the apply kernel --
 //                   {f32 alpha, f32 weight}[nW]
 //                   u16 fix[nF]          read entries that follow a write
@@ -70,6 +70,14 @@ struct __align__(16) RnListHdr {
     uint16_t atW, atR;  // in 16 bytes from the header
 };
 static_assert(sizeof(RnListHdr) == 16, "list header");
+// Shares of the replay.  The read entries of an owner are dealt to the 2^lu thread groups of the apply kernel that have a row
+// each (512 threads, 32 bytes of a row each): unit u gets the reads whose first entry lies in [u q, (u + 1) q), q = ceil(n / 2^lu),
+// a read whole.  run[u] (u q < n) is its first entry.
+__host__ __device__ __forceinline__ int rn_units_log2(int rs) { return 14 - rs; }
+__host__ __device__ __forceinline__ uint32_t rn_runs(uint32_t n, int rs) {  // entries kept for n
+    const uint32_t units = 1u << rn_units_log2(rs);
+    return n < units ? n : units;
+}
 struct RnListAt {  // parts of a list, in 16 bytes from its header
     uint32_t W, R, AW, F, end;
 };
@@ -127,7 +135,18 @@ struct RnListParams {
     // optional, for a short sequence on a state that is updated in place: [bh][owner][2][rn_touch_words] bits of the rows that
     // the call reads or writes and of those that it writes; the others stay in global memory
     uint32_t *touch;
+    // replay of the backward pass (rn_apply.cu)
+    const void *dy;            // upstream gradient of y
+    int64_t dyb, dyh, dyt;
+    float *delta;              // [bh][slice][t][Kw][dcs]: x - row at every write, slices of dcs channels
+    int dcs;
+    float *part;               // [bh][group][t][Kr]: partial dot products, d_r
+    const unsigned char *sched;  // chunk records of the schedule kernel: coefficients of all events
+    int64_t sched_bytes;
+    int sched_L, sched_NEp;
 };
+
+enum { RN_FORWARD = 0, RN_REPLAY = 1 };
 
 // walks the steps of a (b,h): the entry of an owner in step st of block blk; all zero behind the last block
 // (first: this owner's first steps)
@@ -156,3 +175,7 @@ __host__ __device__ __forceinline__ int rn_touch_words(int lr) { return lr < 5 ?
 bool rn_list_plan(int64_t B, int64_t H, int64_t T, int64_t A, int64_t C, int64_t Kw, int64_t Kr, int mass_aware, RnListPlan *pl);
 int rn_launch_lists(const RnListParams &p, const RnListPlan &pl, int dtype, cudaStream_t stream);
 int rn_launch_apply(const RnListParams &p, const RnListPlan &pl, int dtype, cudaStream_t stream);
+// the same for the replay of the backward pass (rn_bwd_lists.cu)
+bool rn_replay_plan(int64_t B, int64_t H, int64_t T, int64_t A, int64_t C, int64_t Kw, int64_t Kr, RnListPlan *pl);
+int rn_launch_replay_lists(const RnListParams &p, const RnListPlan &pl, cudaStream_t stream);
+int rn_launch_replay(const RnListParams &p, const RnListPlan &pl, int dtype, cudaStream_t stream);

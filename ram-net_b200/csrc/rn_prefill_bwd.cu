@@ -3,25 +3,31 @@
 // (packages/ramnet-ops/csrc/ram_attn_ops.cpp:267-310, kernels
 //  packages/ramnet-ops/csrc/ram_attn_segment_parallel.cu:241-416 (replay) and :418-606 (reverse)).
 //
-// Same time-chunk / round structure as the forward pass (rn_prefill.cuh); the chunk records are
+// Same time-chunk / round structure as the general forward path (rn_prefill.cuh); the chunk records are
 // rebuilt by the schedule kernel (which also stores the mass each write found), then
-//   replay   (one CTA per (b,h,channel slice), chunks forward):  re-runs the state, stores
-//            delta = x - slot_before of every write and accumulates d_r = <slot_at_read, d_y>;
-//   reverse  (same mapping, chunks and rounds backward):  carries d_slot in shared memory;
+//   replay   re-runs the state, stores delta = x - slot_before of every write and this channel slice's part of
+//            d_r = <slot_at_read, d_y>: the event-list kernels (rn_bwd_lists.cu, rn_apply.cu) where they fill the chip, else
+//            one CTA per (b,h,channel slice), chunks forward;
+//   reverse  (one CTA per (b,h,channel slice), chunks and rounds backward):  carries d_slot in shared memory;
 //            read:  d_slot[a] += r d_y;   write:  d_gain = <d_slot[a], delta>,
 //            d_x += gain d_slot[a],  d_slot[a] *= 1 - gain;
 //   scalar   (one CTA per (b,h), chunks and rounds backward):  the mass chain: d_w, d_gamma, d_mass.
 // The workspaces of the sweeps are laid out per channel slice, so that a CTA streams through memory of its own:
-// delta as [bh][slice][t][k][channels of the slice] and the partial dot products of a slice (d_r from the replay,
-// d_gain from the reverse sweep) as [bh][slice][t][k]; a reduce kernel adds the slices (fixed order, no atomics).
-#include "rn_prefill.cuh"
+// delta as [bh][slice][t][k][channels of the slice] and the partial dot products of a slice, d_r from the replay and
+// d_gain from the reverse sweep, as [bh][slice][t][k]; a reduce kernel adds the slices (fixed order, no atomics).
+#include <type_traits>
+
+#include "rn_lists.cuh"
 
 struct RnGsuBwdParams {
     RnGsuParams f;            // forward description (idx/val, x, gamma, mask, records, ...)
     const void *dy;           // (B,H,T,C) upstream gradient of y, dtype of x
     int64_t dyb, dyh, dyt;
     float *delta;             // workspace [(bh*nslices + slice)*T + t][Kw][cs]
-    float *part;              // workspace [(bh*nslices + slice)*T + t][Kw + Kr]: d_gain (k < Kw) and d_r partial sums
+    float *part_w;            // workspace [(bh*nslices + slice)*T + t][Kw]: d_gain partial sums
+    float *part_r;            // workspace [(bh*slices_r + slice)*T + t][Kr]: d_r partial sums
+    int slices_r;             // nslices, or the channel groups of the event lists
+    bool lists;               // the replay ran over event lists
     float *dgain;             // workspace [(bh*T + t)*Kw + k], written by the reduce kernel
     float *dval;              // output (B,H,Kw+Kr,T) via strides, zeroed by the caller
     int64_t vb, vh, vk, vt;
@@ -94,6 +100,7 @@ __global__ void __launch_bounds__(RN_APPLY_THREADS, 1) rn_gsu_bwd_sweep_kernel(c
     float *dyt = xt + size_t(L) * CS;
     float *dxlate = dyt + size_t(L) * CS;
 
+    const int PK = REVERSE ? Kw : KT - Kw;  // partial sums a token
     if (tid == 0) {
         rn_mbar_init(&mbar[0], 1);
         rn_mbar_init(&mbar[1], 1);
@@ -153,10 +160,11 @@ __global__ void __launch_bounds__(RN_APPLY_THREADS, 1) rn_gsu_bwd_sweep_kernel(c
         const unsigned char *rec = rec0 + (it & 1) * rec_stride;
         const uint2 *e_pair = reinterpret_cast<const uint2 *>(rec);
         const uint16_t *heads = reinterpret_cast<const uint16_t *>(rec + size_t(NEp) * 8);
-        // this slice's rows of the workspaces: write event (t, k) at (t*Kw + k)*CS in delta, event (t, k) at t*KT + k in part
+        // this slice's rows of the workspaces: write event (t, k) at (t*Kw + k)*CS in delta, write (reverse) or read (replay) k of token t
+        // at t*PK + k in part_w / from t*PK on in part_r
         float *dchunk = bp.delta + ((int64_t(bh) * p.nslices + slice) * p.T + t0) * Kw * CS;
         float *dtok = dchunk + int64_t(tok) * Kw * CS + sub * 4;
-        float *pchunk = bp.part + ((int64_t(bh) * p.nslices + slice) * p.T + t0) * KT;
+        float *pchunk = (REVERSE ? bp.part_w : bp.part_r - Kw) + ((int64_t(bh) * p.nslices + slice) * p.T + t0) * PK;
         if (REVERSE && more && tid == 32) {
             // the deltas of the chunk after this one: one contiguous piece of this slice's workspace
             const int tn = (chunk + step) * L;
@@ -200,7 +208,7 @@ __global__ void __launch_bounds__(RN_APPLY_THREADS, 1) rn_gsu_bwd_sweep_kernel(c
                         late_cf[jb + i] = __uint_as_float(pr[i].x);
                     }
                 } else if (tok_ok && (MODEL || k < KT) && sub == 0 && wr_of(jb + i) == REVERSE) {
-                    pchunk[tok * KT + k] = 0.f;  // a no-op event
+                    pchunk[tok * PK + k] = 0.f;  // a no-op event
                 }
             }
 #pragma unroll
@@ -222,7 +230,7 @@ __global__ void __launch_bounds__(RN_APPLY_THREADS, 1) rn_gsu_bwd_sweep_kernel(c
                     } else {
                         float dot = s.x * dyv.x + s.y * dyv.y + s.z * dyv.z + s.w * dyv.w;
                         dot = rn_group_sum(dot, G, gmask);
-                        if (sub == 0) pchunk[tok * KT + k] = dot;
+                        if (sub == 0) pchunk[tok * PK + k] = dot;
                     }
                 } else {
                     if (!wr_of(jb + i)) {
@@ -233,7 +241,7 @@ __global__ void __launch_bounds__(RN_APPLY_THREADS, 1) rn_gsu_bwd_sweep_kernel(c
                     } else {
                         float dot = s.x * dl[i].x + s.y * dl[i].y + s.z * dl[i].z + s.w * dl[i].w;
                         dot = rn_group_sum(dot, G, gmask);
-                        if (sub == 0) pchunk[tok * KT + k] = dot;
+                        if (sub == 0) pchunk[tok * PK + k] = dot;
                         acc.x = fmaf(cf, s.x, acc.x);
                         acc.y = fmaf(cf, s.y, acc.y);
                         acc.z = fmaf(cf, s.z, acc.z);
@@ -318,7 +326,7 @@ __global__ void __launch_bounds__(RN_APPLY_THREADS, 1) rn_gsu_bwd_sweep_kernel(c
                 const float4 dyr = *reinterpret_cast<const float4 *>(dyt + tok * CS + sub * 4);
                 float dot = v.x * dyr.x + v.y * dyr.y + v.z * dyr.z + v.w * dyr.w;
                 dot = rn_group_sum(dot, G, gmask);
-                if (sub == 0) pchunk[tok * KT + k] = dot;
+                if (sub == 0) pchunk[tok * PK + k] = dot;
             }
             // a token's threads share a warp: none of them goes on to overwrite the token's d_y row for the next chunk
             // while another one still reads it here
@@ -336,7 +344,7 @@ __global__ void __launch_bounds__(RN_APPLY_THREADS, 1) rn_gsu_bwd_sweep_kernel(c
                 if (chan_ok) dl = *reinterpret_cast<const float4 *>(dtok + k * CS);
                 float dot = v.x * dl.x + v.y * dl.y + v.z * dl.z + v.w * dl.w;
                 dot = rn_group_sum(dot, G, gmask);
-                if (sub == 0) pchunk[tok * KT + k] = dot;
+                if (sub == 0) pchunk[tok * PK + k] = dot;
                 acc.x = fmaf(cf, v.x, acc.x);
                 acc.y = fmaf(cf, v.y, acc.y);
                 acc.z = fmaf(cf, v.z, acc.z);
@@ -376,33 +384,55 @@ __global__ void __launch_bounds__(RN_RED_THREADS) rn_gsu_bwd_reduce_kernel(const
     const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H;
     const int t0 = blockIdx.x * RN_RED_TOKENS;
     const int nt = min(RN_RED_TOKENS, p.T - t0);
-    const int Kw = p.Kw, Kr = p.Kr, KT = Kw + Kr;
-    const int64_t slice_stride = int64_t(p.T) * KT;
-    const float *src = bp.part + (int64_t(bh) * p.nslices * p.T + t0) * KT;
-    auto put = [&](const int i, const float sum) {
-        const int t = i / KT, k = i - t * KT;
-        if (k < Kw) bp.dgain[(int64_t(bh) * p.T + t0 + t) * Kw + k] = sum;
-        else red_tile[(k - Kw) * (RN_RED_TOKENS + 1) + t] = sum;
-    };
-    if (((slice_stride | (int64_t(t0) * KT) | (int64_t(nt) * KT)) & 3) == 0) {
-        // four entries per thread and slice: sixteen-byte loads, all slices of an entry requested before the sum
-        for (int i = threadIdx.x * 4; i < nt * KT; i += RN_RED_THREADS * 4) {
-            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-            for (int sl = 0; sl < p.nslices; ++sl) {
-                const float4 v = *reinterpret_cast<const float4 *>(src + sl * slice_stride + i);
-                sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+    const int Kw = p.Kw, Kr = p.Kr;
+    const float *val = p.val + b * p.ib + h * p.ih + int64_t(t0) * p.it;
+    const uint8_t *mask = p.mask ? p.mask + b * p.mb + int64_t(t0) * p.mt : nullptr;
+    const uint32_t magic_w = 0xffffffffu / uint32_t(Kw) + 1u, magic_r = 0xffffffffu / uint32_t(Kr) + 1u;  // i / K == __umulhi(i, magic), i < 4096
+    // d_gain entries of the tokens, then their d_r entries, in one pass so that all loads are in flight together
+    auto sums = [&](auto vec) {
+        constexpr int V = decltype(vec)::value;
+        const int nw = nt * Kw, all = nw + nt * Kr;
+        for (int e = threadIdx.x * V; e < all; e += RN_RED_THREADS * V) {
+            const bool write = e < nw;
+            const int n = write ? Kw : Kr, ns = write ? p.nslices : bp.slices_r, i = write ? e : e - nw;
+            const int64_t slice_stride = int64_t(p.T) * n;
+            const float *src = (write ? bp.part_w : bp.part_r) + (int64_t(bh) * ns * p.T + t0) * n + i;
+            float sum[V];
+#pragma unroll
+            for (int v = 0; v < V; ++v) sum[v] = 0.f;
+            // up to sixteen slices requested before the first is added
+#pragma unroll 1
+            for (int s0 = 0; s0 < ns; s0 += 16, src += 16 * slice_stride) {
+                float part[16][V];
+#pragma unroll
+                for (int sl = 0; sl < 16; ++sl) {
+                    if constexpr (V == 4) {
+                        const float4 v = s0 + sl < ns ? __ldcs(reinterpret_cast<const float4 *>(src + sl * slice_stride)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        part[sl][0] = v.x; part[sl][1] = v.y; part[sl][2] = v.z; part[sl][3] = v.w;
+                    } else {
+                        part[sl][0] = s0 + sl < ns ? src[sl * slice_stride] : 0.f;
+                    }
+                }
+#pragma unroll
+                for (int sl = 0; sl < 16; ++sl)
+#pragma unroll
+                    for (int v = 0; v < V; ++v) sum[v] += part[sl][v];
             }
-            put(i, sum.x); put(i + 1, sum.y); put(i + 2, sum.z); put(i + 3, sum.w);
+            const int t = n == 1 ? i : int(__umulhi(uint32_t(i), write ? magic_w : magic_r)), k = i - t * n;
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                if (write) {
+                    bp.dgain[(int64_t(bh) * p.T + t0 + t) * Kw + k + v] = sum[v];
+                } else {
+                    // the event lists have nothing for a no-op read (zero weight, masked token)
+                    const bool none = bp.lists && (val[int64_t(Kw + k + v) * p.ik + int64_t(t) * p.it] == 0.f || (mask != nullptr && mask[t * p.mt] == 0));
+                    red_tile[(k + v) * (RN_RED_TOKENS + 1) + t] = none ? 0.f : sum[v];
+                }
+            }
         }
-    } else {
-        for (int i = threadIdx.x; i < nt * KT; i += RN_RED_THREADS) {
-            float sum = 0.f;
-#pragma unroll 8
-            for (int sl = 0; sl < p.nslices; ++sl) sum += src[sl * slice_stride + i];
-            put(i, sum);
-        }
-    }
+    };
+    if (((Kw | Kr) & 3) == 0) sums(std::integral_constant<int, 4>{});
+    else sums(std::integral_constant<int, 1>{});
     __syncthreads();
     float *dst = bp.dval + b * bp.vb + h * bp.vh + int64_t(t0) * bp.vt;
     for (int i = threadIdx.x; i < Kr * RN_RED_TOKENS; i += RN_RED_THREADS) {
@@ -601,25 +631,35 @@ __global__ void __launch_bounds__(RN_SCHED_THREADS_MAX) rn_gsu_scalar_bwd_kernel
 // ------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------
+// The event lists cost two launches and a pass over the events before the sweep itself, which takes two thirds of the time of
+// the one in this file (U2 P64 K16 C128 bf16, 128 heads of 16384 tokens: 12.7 ms against 8.2 + 1.2).  So they pay where the
+// sweep is throughput bound: enough CTAs for every SM.
+static bool rn_replay_by_lists(const RnListPlan &lp, int64_t B, int64_t H, int device) {
+    return B * H * lp.ngroups * lp.N >= rn_sm_count(device);
+}
+
 struct RnBwdLayout {
-    size_t off_fwd, off_prev_mass, off_read_mass, off_dgain, off_part, off_delta, total;
+    size_t off_fwd, off_lists, off_prev_mass, off_read_mass, off_dgain, off_part, off_part_r, off_delta, total;
+    bool lists;        // the replay runs over event lists
+    RnListPlan replay;
 };
 
-static void rn_bwd_layout(const RnGsuPlan &pl, int64_t B, int64_t H, int64_t T, int64_t C, int64_t Kw, int64_t Kr,
+static void rn_bwd_layout(const RnGsuPlan &pl, int64_t B, int64_t H, int64_t T, int64_t A, int64_t C, int64_t Kw, int64_t Kr, int device,
                           RnBwdLayout *lo) {
+    lo->lists = rn_replay_plan(B, H, T, A, C, Kw, Kr, &lo->replay) && rn_replay_by_lists(lo->replay, B, H, device);
     size_t off = 0;
-    lo->off_fwd = off;
-    off = rn_align(off + pl.total, 256);
-    lo->off_prev_mass = off;
-    off = rn_align(off + size_t(B * H * T * Kw) * 4, 256);
-    lo->off_read_mass = off;
-    off = rn_align(off + size_t(B * H * T * Kr) * 4, 256);
-    lo->off_dgain = off;
-    off = rn_align(off + size_t(B * H * T * Kw) * 4, 256);
-    lo->off_part = off;
-    off = rn_align(off + size_t(B * H * T * (Kw + Kr)) * size_t(pl.nslices) * 4, 256);
-    lo->off_delta = off;
-    off = rn_align(off + size_t(B * H * T * Kw) * size_t(pl.nslices) * size_t(pl.cs) * 4, 256);
+    auto take = [&](size_t *at, size_t bytes) {
+        *at = off;
+        off = rn_align(off + bytes, 256);
+    };
+    take(&lo->off_fwd, pl.total);
+    take(&lo->off_lists, lo->lists ? lo->replay.total : 0);
+    take(&lo->off_prev_mass, size_t(B * H * T * Kw) * 4);
+    take(&lo->off_read_mass, size_t(B * H * T * Kr) * 4);
+    take(&lo->off_dgain, size_t(B * H * T * Kw) * 4);
+    take(&lo->off_part, size_t(B * H * T * Kw) * size_t(pl.nslices) * 4);
+    take(&lo->off_part_r, size_t(B * H * T * Kr) * size_t(lo->lists ? lo->replay.ngroups : pl.nslices) * 4);
+    take(&lo->off_delta, size_t(B * H * T * Kw) * size_t(pl.nslices) * size_t(pl.cs) * 4);
     lo->total = off;
 }
 
@@ -629,7 +669,7 @@ extern "C" int64_t rn_gsu_bwd_workspace_bytes(int64_t B, int64_t H, int64_t T, i
     RnGsuPlan pl;
     if (rn_gsu_plan(B, H, T, A, C, Kw, Kr, device, &pl, 1)) return -1;
     RnBwdLayout lo;
-    rn_bwd_layout(pl, B, H, T, C, Kw, Kr, &lo);
+    rn_bwd_layout(pl, B, H, T, A, C, Kw, Kr, device, &lo);
     return int64_t(lo.total);
 }
 
@@ -681,13 +721,19 @@ static int rn_launch_scalar_bwd(const RnGsuBwdParams &bp, const RnGsuPlan &pl, s
 }
 
 template <typename T>
-static int rn_run_bwd(const RnGsuBwdParams &bp, const RnGsuPlan &pl, int dtype, cudaStream_t stream) {
+static int rn_run_bwd(const RnGsuBwdParams &bp, const RnListParams &replay, const RnGsuPlan &pl, const RnBwdLayout &lo, int dtype,
+                      cudaStream_t stream) {
     rn_prof_reset();
     rn_prof_mark(stream);
     if (int rc = rn_gsu_launch_schedule(bp.f, pl, dtype, stream)) return rc;
     RN_CUDA(cudaGetLastError());
     rn_prof_mark(stream);
-    if (int rc = rn_launch_sweep<T, false>(bp, pl, stream)) return rc;
+    if (lo.lists) {
+        if (int rc = rn_launch_replay_lists(replay, lo.replay, stream)) return rc;
+        if (int rc = rn_launch_replay(replay, lo.replay, dtype, stream)) return rc;
+    } else if (int rc = rn_launch_sweep<T, false>(bp, pl, stream)) {
+        return rc;
+    }
     RN_CUDA(cudaGetLastError());
     rn_prof_mark(stream);
     if (int rc = rn_launch_sweep<T, true>(bp, pl, stream)) return rc;
@@ -740,7 +786,7 @@ extern "C" int rn_gsu_bwd(const int32_t *idx, const float *val, const int64_t *i
                      dx_strides[0] | dx_strides[1] | dx_strides[2]) & 3) == 0,
                "x, d_y and d_x must be aligned to 4 elements (pointer and strides)");
     RnBwdLayout lo;
-    rn_bwd_layout(pl, B, H, T, C, Kw, Kr, &lo);
+    rn_bwd_layout(pl, B, H, T, A, C, Kw, Kr, device, &lo);
     RN_REQUIRE(workspace_bytes >= int64_t(lo.total), "workspace too small: %lld < %lld bytes", (long long)workspace_bytes,
                (long long)lo.total);
     RN_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "workspace must be 256-byte aligned");
@@ -780,7 +826,10 @@ extern "C" int rn_gsu_bwd(const int32_t *idx, const float *val, const int64_t *i
     bp.dy = d_y; bp.dyb = dy_strides[0]; bp.dyh = dy_strides[1]; bp.dyt = dy_strides[2];
     bp.delta = reinterpret_cast<float *>(ws + lo.off_delta);
     bp.dgain = reinterpret_cast<float *>(ws + lo.off_dgain);
-    bp.part = reinterpret_cast<float *>(ws + lo.off_part);
+    bp.part_w = reinterpret_cast<float *>(ws + lo.off_part);
+    bp.part_r = reinterpret_cast<float *>(ws + lo.off_part_r);
+    bp.lists = lo.lists;
+    bp.slices_r = lo.lists ? lo.replay.ngroups : pl.nslices;
     bp.dval = d_val; bp.vb = dval_strides[0]; bp.vh = dval_strides[1]; bp.vk = dval_strides[2]; bp.vt = dval_strides[3];
     bp.dx = d_x; bp.dxb = dx_strides[0]; bp.dxh = dx_strides[1]; bp.dxt = dx_strides[2];
     bp.dgamma = d_gamma;
@@ -789,7 +838,30 @@ extern "C" int rn_gsu_bwd(const int32_t *idx, const float *val, const int64_t *i
 
     RN_REQUIRE(pl.smem_tables, "the backward pass needs the per-head mass table to fit shared memory (A=%lld)", (long long)A);
 
-    if (dtype == RN_F32) return rn_run_bwd<float>(bp, pl, dtype, stream);
-    if (dtype == RN_F16) return rn_run_bwd<__half>(bp, pl, dtype, stream);
-    return rn_run_bwd<__nv_bfloat16>(bp, pl, dtype, stream);
+    RnListParams q{};
+    if (lo.lists) {
+        const RnListPlan &lp = lo.replay;
+        q.idx = idx; q.val = val;
+        q.ib = p.ib; q.ih = p.ih; q.ik = p.ik; q.it = p.it;
+        q.mask = mask; q.mb = p.mb; q.mt = p.mt;
+        q.x = x; q.xb = p.xb; q.xh = p.xh; q.xt = p.xt;
+        q.dy = d_y; q.dyb = bp.dyb; q.dyh = bp.dyh; q.dyt = bp.dyt;
+        q.slot_in = slot_in;
+        q.B = p.B; q.H = p.H; q.T = p.T; q.A = p.A; q.C = p.C; q.Kw = p.Kw; q.Kr = p.Kr;
+        q.L = lp.L; q.nblocks = lp.nblocks; q.lg = lp.lg; q.lr = lp.lr; q.ngroups = lp.ngroups; q.capR = lp.capR; q.capW = lp.capW;
+        q.blk_bytes = lp.blk_bytes; q.list_max = lp.list_max; q.whole_max = lp.whole_max; q.step_max = lp.step_max;
+        q.a_magic = 0xffffffffu / uint32_t(A);
+        q.rs = lp.cs == 32 ? 7 : 6;
+        q.status = p.status;
+        q.recs = ws + lo.off_lists;
+        q.first = reinterpret_cast<uint4 *>(q.recs + lp.off_first);
+        q.delta = bp.delta;
+        q.dcs = pl.cs;
+        q.part = bp.part_r;
+        q.sched = p.records; q.sched_bytes = p.rec_bytes; q.sched_L = p.L; q.sched_NEp = p.NEp;
+    }
+
+    if (dtype == RN_F32) return rn_run_bwd<float>(bp, q, pl, lo, dtype, stream);
+    if (dtype == RN_F16) return rn_run_bwd<__half>(bp, q, pl, lo, dtype, stream);
+    return rn_run_bwd<__nv_bfloat16>(bp, q, pl, lo, dtype, stream);
 }
