@@ -269,17 +269,20 @@ struct RamAttention : public torch::autograd::Function<RamAttention> {
         at::AutoDispatchBelowADInplaceOrView below;
         if (!dy.defined()) dy = at::zeros({c.B, c.T, c.H, c.C}, x.options());
         if (!rows_of_four(dy)) dy = dy.contiguous();
-        const auto f32 = x.options().dtype(at::kFloat);
-        const Tensor slot_in = slot.defined() ? slot : at::zeros({c.B, c.H, c.A, c.C}, f32);
-        const Tensor mass_in = mass.defined() ? mass : at::full({c.B, c.H, c.A}, c.mass_init, f32);
-        dslot_post = dslot_post.defined() ? dslot_post.contiguous() : at::zeros({c.B, c.H, c.A, c.C}, f32);
-        dmass_post = dmass_post.defined() ? dmass_post.contiguous() : at::zeros({c.B, c.H, c.A}, f32);
+        if (dslot_post.defined()) dslot_post = dslot_post.contiguous();
+        if (dmass_post.defined()) dmass_post = dmass_post.contiguous();
+        const bool want_dslot = slot.defined() && ctx->needs_input_grad(4), want_dmass = mass.defined() && ctx->needs_input_grad(5);
 
         const int64_t K = c.Kw + c.Kr;
-        Tensor dval = at::zeros({c.B, c.T, c.H, K}, f32);
+        Tensor dval = empty({c.B, c.T, c.H, K}, at::kFloat, c.device);
         Tensor dx = empty({c.B, c.T, c.H, c.C}, x.scalar_type(), c.device);
         Tensor dgamma = empty({c.B, c.H, c.T}, at::kFloat, c.device);
-        Tensor dslot = empty({c.B, c.H, c.A, c.C}, at::kFloat, c.device), dmass = empty({c.B, c.H, c.A}, at::kFloat, c.device);
+        // the state and its gradients where they exist; a state that was not given is zeros and mass_init, gradients that did not
+        // come are zeros
+        Tensor dslot, dmass;
+        if (want_dslot) dslot = empty({c.B, c.H, c.A, c.C}, at::kFloat, c.device);
+        if (want_dmass) dmass = empty({c.B, c.H, c.A}, at::kFloat, c.device);
+        auto in = [](const Tensor &v) { return v.defined() ? v.const_data_ptr<float>() : nullptr; };
         const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(c.device.index());
         const int64_t bytes = rn_gsu_bwd_workspace_bytes(c.B, c.H, c.T, c.A, c.C, c.Kw, c.Kr, c.device.index());
         TORCH_CHECK(bytes >= 0, rn_last_error());
@@ -287,12 +290,12 @@ struct RamAttention : public torch::autograd::Function<RamAttention> {
         const int64_t sv[4] = {c.T * c.H * K, K, 1, c.H * K};
         const Rows sx(x), sg(gamma), sdy(dy), sdx(dx);
         const int64_t sm[2] = {c.mask.defined() ? c.mask.stride(0) : 0, c.mask.defined() ? c.mask.stride(1) : 0};
-        check(rn_gsu_bwd(idx.const_data_ptr<int32_t>(), val.const_data_ptr<float>(), sv, x.const_data_ptr(), sx.s, gamma.const_data_ptr(),
-                         sg.s, c.code, c.mask_ptr(), sm, slot_in.const_data_ptr<float>(), mass_in.const_data_ptr<float>(), dy.const_data_ptr(),
-                         sdy.s, dslot_post.const_data_ptr<float>(), dmass_post.const_data_ptr<float>(), dval.mutable_data_ptr<float>(), sv,
-                         dx.mutable_data_ptr(), sdx.s, dgamma.mutable_data_ptr<float>(), dslot.mutable_data_ptr<float>(),
-                         dmass.mutable_data_ptr<float>(), ws.mutable_data_ptr(), ws.numel(), c.B, c.H, c.T, c.A, c.C, c.Kw, c.Kr, c.mass_aware,
-                         c.eps, c.device.index(), stream));
+        check(rn_gsu_bwd_init(idx.const_data_ptr<int32_t>(), val.const_data_ptr<float>(), sv, x.const_data_ptr(), sx.s,
+                              gamma.const_data_ptr(), sg.s, c.code, c.mask_ptr(), sm, in(slot), in(mass), c.mass_init, dy.const_data_ptr(),
+                              sdy.s, in(dslot_post), in(dmass_post), dval.mutable_data_ptr<float>(), sv, dx.mutable_data_ptr(), sdx.s,
+                              dgamma.mutable_data_ptr<float>(), want_dslot ? dslot.mutable_data_ptr<float>() : nullptr,
+                              want_dmass ? dmass.mutable_data_ptr<float>() : nullptr, ws.mutable_data_ptr(), ws.numel(), c.B, c.H, c.T,
+                              c.A, c.C, c.Kw, c.Kr, c.mass_aware, c.eps, c.device.index(), stream));
         if (ctx->needs_input_grad(0) || ctx->needs_input_grad(1)) {
             Tensor dw = empty({c.B, c.T, c.H, c.U, c.P}, w.scalar_type(), c.device), dr = empty({c.B, c.T, c.H, c.U, c.P}, w.scalar_type(), c.device);
             int64_t sa[5], sd[5];
@@ -307,8 +310,8 @@ struct RamAttention : public torch::autograd::Function<RamAttention> {
         }
         if (ctx->needs_input_grad(2)) out[2] = dx;
         if (ctx->needs_input_grad(3)) out[3] = dgamma.permute({0, 2, 1}).to(gamma.scalar_type());
-        if (slot.defined() && ctx->needs_input_grad(4)) out[4] = dslot;
-        if (mass.defined() && ctx->needs_input_grad(5)) out[5] = dmass;
+        if (want_dslot) out[4] = dslot;
+        if (want_dmass) out[5] = dmass;
         return out;
     }
 };

@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(RN_SCHED_THREADS_MAX) rn_gsu_schedule_kernel(c
         // chain heads (the events that retired in the second claim round, er == 1) in any order: warp-aggregated append
 #pragma unroll
         for (int j = 0; j < EPT; ++j) {
-            const bool emit = er[j] == 1;
+            const bool emit = p.pairs && er[j] == 1;
             const unsigned act = __ballot_sync(RN_FULL, emit);
             if (act != 0u) {
                 const int lane = tid & 31, leader = __ffs(act) - 1;
@@ -222,14 +222,16 @@ __global__ void __launch_bounds__(RN_SCHED_THREADS_MAX) rn_gsu_schedule_kernel(c
                 const bool dead = er[j] < 0;
                 o_meta[e] = rn_ev_pack(ea[j], dead ? 0 : er[j], dead);
                 o_coef[e] = dead ? 0.f : ec[j];
-                uint32_t link = RN_LINK_DEAD;
-                if (!dead) {
-                    const uint32_t kind = er[j] == 0 ? RN_KIND_FIRST : (er[j] == 1 ? RN_KIND_HEAD : RN_KIND_LATER);
-                    link = (rn_row_of_slot(ea[j], A, p.row_shift) & 0xffffu) | (kind << RN_LINK_KIND_SHIFT);
-                    const uint32_t nx = SMEM_TABLES ? nxt[e] : 0xffffu;
-                    if (nx != 0xffffu) link |= RN_LINK_NEXT | (nx << 16);
+                if (p.pairs) {
+                    uint32_t link = RN_LINK_DEAD;
+                    if (!dead) {
+                        const uint32_t kind = er[j] == 0 ? RN_KIND_FIRST : (er[j] == 1 ? RN_KIND_HEAD : RN_KIND_LATER);
+                        link = (rn_row_of_slot(ea[j], A, p.row_shift) & 0xffffu) | (kind << RN_LINK_KIND_SHIFT);
+                        const uint32_t nx = SMEM_TABLES ? nxt[e] : 0xffffu;
+                        if (nx != 0xffffu) link |= RN_LINK_NEXT | (nx << 16);
+                    }
+                    o_pair[e] = make_uint2(__float_as_uint(dead ? 0.f : ec[j]), link);
                 }
-                o_pair[e] = make_uint2(__float_as_uint(dead ? 0.f : ec[j]), link);
                 if (p.wide) o_slot[e] = ea[j];
             }
         }
@@ -268,7 +270,7 @@ __global__ void __launch_bounds__(RN_SCHED_THREADS_MAX) rn_gsu_schedule_kernel(c
         }
         __syncthreads();  // n_heads / n_rheads are complete
         if (tid == 0) {
-            o_heads[0] = uint16_t(n_heads);
+            if (p.pairs) o_heads[0] = uint16_t(n_heads);
             if (SMEM_TABLES && p.reverse)
                 reinterpret_cast<uint16_t *>(rec + RN_GSU_HDR_BYTES + size_t(NEp) * 25 + 16)[0] = uint16_t(n_rheads);
         }
@@ -287,7 +289,7 @@ __global__ void __launch_bounds__(RN_SCHED_THREADS_MAX) rn_gsu_schedule_kernel(c
         __syncthreads();  // gam / tok_live of the next chunk are complete; ev_v / ev_c may be reused
     }
 
-    if (SMEM_TABLES) {
+    if (SMEM_TABLES && p.mass_out != nullptr) {
         float *mass_out = p.mass_out + int64_t(bh) * A;
         for (int a = tid; a < A; a += NT) mass_out[a] = mass[a];
     }

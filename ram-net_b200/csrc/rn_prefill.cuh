@@ -111,7 +111,8 @@ struct RnGsuParams {
     uint32_t *claim;          // global claim table (B*H*A) when the tables do not fit shared memory
     float *prev_mass;         // optional: mass of the slot before each write, [(bh*T + t)*Kw + k] (backward)
     float *read_mass;         // optional: mass of the slot at each read, [(bh*T + t)*Kr + k] (mass-aware backward)
-    int reverse;              // also emit the backward pairs / heads of every chunk
+    int pairs;                // emit the pairs / heads of every chunk (replay of rn_prefill_bwd.cu)
+    int reverse;              // and their mirror image, for its reverse sweep
     int row_shift;            // rn_row_of_slot
     // apply kernel
     int cs;                   // channels per CTA (multiple of 4)

@@ -29,15 +29,15 @@ struct RnGsuBwdParams {
     int slices_r;             // nslices, or the channel groups of the event lists
     bool lists;               // the replay ran over event lists
     float *dgain;             // workspace [(bh*T + t)*Kw + k], written by the reduce kernel
-    float *dval;              // output (B,H,Kw+Kr,T) via strides, zeroed by the caller
+    float *dval;              // output (B,H,Kw+Kr,T) via strides
     int64_t vb, vh, vk, vt;
     void *dx;                 // output (B,H,T,C), dtype of x
     int64_t dxb, dxh, dxt;
     float *dgamma;            // output (B,H,T) contiguous fp32
-    const float *dslot_post;  // (B,H,A,C)
-    float *dslot_out;
-    const float *dmass_post;  // (B,H,A)
-    float *dmass_out;
+    const float *dslot_post;  // (B,H,A,C), null: zeros
+    float *dslot_out;         // null: not wanted
+    const float *dmass_post;  // (B,H,A), null: zeros
+    float *dmass_out;         // null: not wanted
     float *dmass_ws;          // global d_mass table when it does not fit shared memory (aliases dmass_out)
 };
 
@@ -121,11 +121,12 @@ __global__ void __launch_bounds__(RN_APPLY_THREADS, 1) rn_gsu_bwd_sweep_kernel(c
     bool failed = false;
     if (tid == 0) fetch(0, first);
     {
-        const float *src = (REVERSE ? bp.dslot_post : p.slot_in) + int64_t(bh) * A * C + c0;
+        const float *state = REVERSE ? bp.dslot_post : p.slot_in;  // null: zeros
+        const float *src = state + int64_t(bh) * A * C + c0;
         for (int i = tid; i < A * G; i += RN_APPLY_THREADS) {
             const int a = i / G, sg = i - a * G;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (sg * 4 < cvalid) v = *reinterpret_cast<const float4 *>(src + int64_t(a) * C + sg * 4);
+            if (state != nullptr && sg * 4 < cvalid) v = *reinterpret_cast<const float4 *>(src + int64_t(a) * C + sg * 4);
             *reinterpret_cast<float4 *>(S + rn_row_of_slot(uint32_t(a), A, p.row_shift) * CS + sg * 4) = v;
         }
     }
@@ -360,7 +361,7 @@ __global__ void __launch_bounds__(RN_APPLY_THREADS, 1) rn_gsu_bwd_sweep_kernel(c
         }
     }
 
-    if (REVERSE) {
+    if (REVERSE && bp.dslot_out != nullptr) {
         __syncthreads();
         float *dst = bp.dslot_out + int64_t(bh) * A * C + c0;
         for (int i = tid; i < A * G; i += RN_APPLY_THREADS) {
@@ -482,9 +483,9 @@ __global__ void __launch_bounds__(RN_SCHED_THREADS_MAX) rn_gsu_scalar_bwd_kernel
     float *rd_u = dg_term + size_t(p.L) * Kw;
     float *rd_r = rd_u + size_t(p.L) * Kr;
     float *rd_dot = rd_r + size_t(p.L) * Kr;
-    const float *src = bp.dmass_post + int64_t(bh) * A;
+    const float *src = bp.dmass_post ? bp.dmass_post + int64_t(bh) * A : nullptr;
     for (int a = tid; a < A; a += NT)
-        if (SMEM_TABLE || src != dmass) dmass[a] = src[a];
+        if (SMEM_TABLE || src != dmass) dmass[a] = src ? src[a] : 0.f;
 
     int ev_t[EPT], ev_k[EPT];
 #pragma unroll
@@ -561,6 +562,8 @@ __global__ void __launch_bounds__(RN_SCHED_THREADS_MAX) rn_gsu_scalar_bwd_kernel
             er[j] = -1;
             ea[j] = 0;
             ew[j] = em[j] = eg[j] = 0.f;
+            if ((cur[j].meta & RN_EV_DEAD) && ev_t[j] < Lc && j * NT + tid < NEp && ev_k[j] < Kw)  // a no-op write
+                bp.dval[b * bp.vb + h * bp.vh + int64_t(ev_k[j]) * bp.vk + int64_t(t0 + ev_t[j]) * bp.vt] = 0.f;
             if (!(cur[j].meta & RN_EV_DEAD)) {
                 er[j] = rn_ev_round(cur[j].meta);
                 ea[j] = pow2 ? uint32_t(cur[j].raw & (A - 1)) : uint32_t(cur[j].raw % A);
@@ -622,7 +625,7 @@ __global__ void __launch_bounds__(RN_SCHED_THREADS_MAX) rn_gsu_scalar_bwd_kernel
         }
         __syncthreads();
     }
-    if (SMEM_TABLE) {
+    if (SMEM_TABLE && bp.dmass_out != nullptr) {
         float *dst = bp.dmass_out + int64_t(bh) * A;
         for (int a = tid; a < A; a += NT) dst[a] = dmass[a];
     }
@@ -769,9 +772,23 @@ extern "C" int rn_gsu_bwd(const int32_t *idx, const float *val, const int64_t *i
                           int64_t T, int64_t A, int64_t C, int64_t Kw, int64_t Kr, int mass_aware, double eps, int device,
                           void *stream_) {
     rn_clear_error();
-    RN_REQUIRE(idx && val && idx_strides && x && x_strides && gamma && gamma_strides && slot_in && mass_in && d_y &&
-                   dy_strides && d_slot_post && d_mass_post && d_val && dval_strides && d_x && dx_strides && d_gamma &&
-                   d_slot && d_mass && workspace,
+    RN_REQUIRE(slot_in && mass_in && d_slot_post && d_mass_post && d_slot && d_mass, "null pointer argument");
+    return rn_gsu_bwd_init(idx, val, idx_strides, x, x_strides, gamma, gamma_strides, dtype, mask, mask_strides, slot_in, mass_in, 0.0,
+                           d_y, dy_strides, d_slot_post, d_mass_post, d_val, dval_strides, d_x, dx_strides, d_gamma, d_slot, d_mass,
+                           workspace, workspace_bytes, B, H, T, A, C, Kw, Kr, mass_aware, eps, device, stream_);
+}
+
+extern "C" int rn_gsu_bwd_init(const int32_t *idx, const float *val, const int64_t *idx_strides, const void *x,
+                               const int64_t *x_strides, const void *gamma, const int64_t *gamma_strides, int dtype,
+                               const uint8_t *mask, const int64_t *mask_strides, const float *slot_in, const float *mass_in,
+                               double mass_init, const void *d_y, const int64_t *dy_strides, const float *d_slot_post,
+                               const float *d_mass_post, float *d_val, const int64_t *dval_strides, void *d_x,
+                               const int64_t *dx_strides, float *d_gamma, float *d_slot, float *d_mass, void *workspace,
+                               int64_t workspace_bytes, int64_t B, int64_t H, int64_t T, int64_t A, int64_t C, int64_t Kw,
+                               int64_t Kr, int mass_aware, double eps, int device, void *stream_) {
+    rn_clear_error();
+    RN_REQUIRE(idx && val && idx_strides && x && x_strides && gamma && gamma_strides && d_y && dy_strides && d_val && dval_strides &&
+                   d_x && dx_strides && d_gamma && workspace,
                "null pointer argument");
     RN_REQUIRE(dtype == RN_F32 || dtype == RN_F16 || dtype == RN_BF16, "unsupported dtype code %d", dtype);
     RN_REQUIRE(x_strides[3] == 1 && dy_strides[3] == 1 && dx_strides[3] == 1, "Tensor x / d_y / d_x last dim must be contiguous");
@@ -803,7 +820,7 @@ extern "C" int rn_gsu_bwd(const int32_t *idx, const float *val, const int64_t *i
     p.gamma = gamma; p.gb = gamma_strides[0]; p.gh = gamma_strides[1]; p.gt = gamma_strides[2];
     p.mask = mask;
     if (mask) { p.mb = mask_strides[0]; p.mt = mask_strides[1]; }
-    p.slot_in = slot_in; p.mass_in = mass_in;
+    p.slot_in = slot_in; p.mass_in = mass_in; p.mass_init = float(mass_init);
     p.B = int(B); p.H = int(H); p.T = int(T); p.A = int(A); p.C = int(C); p.Kw = int(Kw); p.Kr = int(Kr);
     p.L = pl.L; p.nchunks = pl.nchunks; p.NE = pl.NE; p.NEp = pl.NEp;
     p.row_shift = rn_row_shift(A);
@@ -817,6 +834,7 @@ extern "C" int rn_gsu_bwd(const int32_t *idx, const float *val, const int64_t *i
     p.claim = reinterpret_cast<uint32_t *>(fws + pl.off_claim);
     p.cs = pl.cs; p.nslices = pl.nslices; p.state_in_smem = pl.state_in_smem;
     p.reverse = 1;
+    p.pairs = !lo.lists;
     p.prev_mass = reinterpret_cast<float *>(ws + lo.off_prev_mass);
     p.read_mass = mass_aware ? reinterpret_cast<float *>(ws + lo.off_read_mass) : nullptr;
     // the schedule kernel writes the final mass somewhere: d_mass doubles as that scratch before
@@ -829,6 +847,7 @@ extern "C" int rn_gsu_bwd(const int32_t *idx, const float *val, const int64_t *i
     bp.part_w = reinterpret_cast<float *>(ws + lo.off_part);
     bp.part_r = reinterpret_cast<float *>(ws + lo.off_part_r);
     bp.lists = lo.lists;
+    RN_REQUIRE(d_mass != nullptr || size_t(A) * 4 + size_t(pl.L) * (Kw + 3 * Kr) * 4 <= 200 * 1024, "d_mass must be given for this many slots");
     bp.slices_r = lo.lists ? lo.replay.ngroups : pl.nslices;
     bp.dval = d_val; bp.vb = dval_strides[0]; bp.vh = dval_strides[1]; bp.vk = dval_strides[2]; bp.vt = dval_strides[3];
     bp.dx = d_x; bp.dxb = dx_strides[0]; bp.dxh = dx_strides[1]; bp.dxt = dx_strides[2];
