@@ -243,7 +243,7 @@ def run_prefill(args, device, rank, barrier, max_over_ranks, batch=None, full=Tr
         y_sample = y_dev.permute(0, 2, 1, 3)[0:1, :PARITY_TOKENS, h0:h1].float().cpu()   # (1, T', 4, C)
     keep.clear()
     names = ["rn_addr_fast_kernel"] + (["rn_gsu_owner_kernel"] if len(t_gsu[0]) == 1 else
-                                       ["rn_gsu_schedule_kernel", "rn_gsu_apply_fast_kernel"])
+                                       ["rn_lists_kernel", "rn_gains_kernel", "rn_apply_kernel"])
     kms = [median(t_addr)] + [median([t[i] for t in t_gsu]) for i in range(len(t_gsu[0]))]
     result = dict(tokens_per_pass=B * T, regions_ms=regions, passes=args.steps * passes_per_step,
                   passes_per_step=passes_per_step, clocks=clocks.summary(), kernels=dict(zip(names, kms)),
@@ -966,8 +966,6 @@ def main():
 # case, per (b,t,h), to be scaled to the benchmark shape by the token-heads processed (the traffic is x / y rows,
 # decoded addresses and the state round trip, all proportional to them at fixed T).  None: no capture yet.
 TRAFFIC = {
-    "rn_gsu_apply_fast_kernel": {"bytes_per_bth": (139.20384e6 + 63.06048e6) / (2 * 4096 * 16),
-                                 "capture": "ncu, --ncu-case prefill_small (B2 T4096 H16), scaled by token-heads"},
 }
 
 

@@ -533,7 +533,7 @@ extern "C" int64_t rn_gsu_workspace_bytes(int64_t B, int64_t H, int64_t T, int64
 }
 
 // Which kernels a prefill call of this shape runs, for tests and benchmarks that must prove they exercise the
-// same template instances: out[0] = 1 fast apply kernel / 0 general, out[1] = channels per CTA, out[2] = events
+// same template instances: out[0] = 1 shape of the backward sweeps / 0 not, out[1] = channels per CTA, out[2] = events
 // per thread (forward), out[3] = channel slices, out[4] = chunk length, out[5] = state slice in shared memory,
 // out[6] = events per thread (backward sweeps), out[7] = schedule tables in shared memory.
 extern "C" int rn_gsu_plan_info(int64_t B, int64_t H, int64_t T, int64_t A, int64_t C, int64_t Kw, int64_t Kr, int reverse,
@@ -676,7 +676,7 @@ extern "C" int rn_gsu_fwd_init(const int32_t *idx, const float *val, const int64
         // rc < 0: this device cannot keep a 16-CTA cluster of that size resident; use the channel-slice kernels
     }
     const size_t esz = dtype == RN_F32 ? 4 : 2;
-    // the list kernels and the fast apply kernel move x / y in 4-element vectors
+    // the list kernels move x / y in 4-element vectors
     const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & (4 * esz - 1)) == 0 &&
                          ((x_strides[0] | x_strides[1] | x_strides[2] | y_strides[0] | y_strides[1] | y_strides[2]) & 3) == 0;
     RnListPlan lp;

@@ -4,17 +4,15 @@
 // or one read of one slot) gets a ROUND number: the count of earlier live events of the same
 // chunk on the same slot (writes of a token come before its reads).  Events of one round touch
 // pairwise different slots, so a round is applied by all threads in parallel with no atomics;
-// rounds are separated by barriers.  Two kernels:
+// rounds are separated by barriers.  The event-list kernels (rn_lists.cuh) are the forward path of most shapes; this one remains for
+// the others (C not a multiple of 4, more than 16384 slots, unaligned rows), and its schedule for the backward pass.
 //
 //   schedule (one CTA per (b,h), chunks in order):   rounds, the mass recurrence and the gain
-//       of every write, the (mass-aware) coefficient of every read -> one record per chunk with
-//       the events sorted by round.  Channel independent, so done once per (b,h).
-//   apply (one CTA per (b,h, channel slice)):   the slice [A][cs] of the slot state stays in
-//       shared memory for the whole sequence; the chunk records are streamed into shared memory
-//       with 1-D bulk async copies (TMA, mbarrier completion) one chunk ahead; per chunk the
-//       rounds are applied (row update / row read into a per-(token,k) buffer), the reads are
-//       reduced over k in a fixed order and y is stored.  Deterministic: no floating-point
-//       atomics anywhere.
+//       of every write, the (mass-aware) coefficient of every read -> one record per chunk.
+//       Channel independent, so done once per (b,h).
+//   apply (one CTA per (b,h, channel slice)):   per chunk the rounds are applied (row update / row read into a
+//       per-(token,k) buffer), the reads are reduced over k in a fixed order and y is stored.  Deterministic: no
+//       floating-point atomics anywhere.
 //
 // Chunk record (global workspace, 16-byte aligned, fixed size per call); entry e = t * (Kw+Kr) + k
 // keeps the order of the decoded addresses, so the record is written and read coalesced:
@@ -22,7 +20,7 @@
 //   u32 meta[NEp]:  bits 0-15 slot (narrow format, A <= 65536), 16-23 round, 24 dead (no-op event:
 //                   zero weight or masked token)
 //   f32 coef[NEp]:  gain of a write / weight of a read (mass-aware scaling folded in)
-//   {f32 coef, u32 link}[NEp]:  the same coefficient next to the event's link word: bits 0-15 row of the
+//   {f32 coef, u32 link}[NEp]:  (for the replay of the backward pass) the same coefficient next to the event's link word: bits 0-15 row of the
 //                   slot in the shared-memory slice (rn_row_of_slot),
 //                   16-27 the following live event of the chunk on the same slot, 28-29 kind (0 first
 //                   event of its slot in the chunk, 2 second event = head of the slot's chain,
@@ -38,8 +36,8 @@
 //                   chain), 3 = earlier
 //   u16 heads[8 + NEp/2]:  the backward chain heads
 // The first events (~80 % of a chunk) are applied token-major (dense).  The later events of a slot
-// form a chain (head, then link by link); the fast apply kernel walks a chain with the slot row in
-// registers.  The backward sweeps and the general apply kernel go round by round over meta[]
+// form a chain (head, then link by link); the backward sweeps walk a chain with the slot row in
+// registers.  The general apply kernel and the mass chain of the backward pass go round by round over meta[]
 // instead.
 #pragma once
 
@@ -137,9 +135,9 @@ struct RnGsuPlan {
     int wide;              // A > 65536: records carry a separate slot array
     int64_t rec_bytes;
     int reverse;           // records carry the backward links
-    int fast;              // fast apply kernel (C % 4 == 0, narrow records, state in shared memory)
-    int tpt_log2, ev;      // fast apply kernel: threads per token, events per thread
-    int tptb_log2, evb;    // backward sweep kernels (RN_SWEEP_THREADS threads)
+    int fast;              // shapes of the backward sweeps (C % 4 == 0, narrow records, state in shared memory)
+    int tpt_log2, ev;      // backward sweep kernels: threads per token, events per thread
+    int tptb_log2, evb;    // the same with RN_SWEEP_THREADS threads
     int cs, nslices, state_in_smem;
     size_t apply_smem;
     // workspace layout (byte offsets)

@@ -47,7 +47,7 @@ __device__ __forceinline__ float rn_group_sum(float v, int G, unsigned mask) {
 }
 
 // ------------------------------------------------------------------------------------------
-// replay / reverse kernels: same organisation as rn_gsu_apply_fast_kernel
+// replay / reverse kernels
 // ------------------------------------------------------------------------------------------
 // One 1024-thread CTA per (b,h, channel slice); the slice of the slot state (replay) or of its gradient
 // (reverse) stays in shared memory; the {coef, link} pairs and the chain heads of a chunk arrive by a
@@ -61,7 +61,7 @@ __device__ __forceinline__ float rn_group_sum(float v, int G, unsigned mask) {
 //            write: this slice's part of d_gain = <d_slot, delta>, d_x += gain * d_slot, d_slot *= 1 - gain
 // Every (token, k) of a chunk gets its partial dot product from exactly one thread (zero for a no-op event), so the
 // partial sums need no clearing.
-// MODEL: the instance for Kw = Kr = 16 with 64-token chunks (see rn_gsu_apply_fast_kernel)
+// MODEL: the instance for Kw = Kr = 16 with 64-token chunks
 template <typename T, int CS, int EV, bool REVERSE, bool MODEL = false>
 __global__ void __launch_bounds__(RN_APPLY_THREADS, 1) rn_gsu_bwd_sweep_kernel(const RnGsuBwdParams bp, const int tpt_log2_) {
     constexpr int G = CS / 4;
