@@ -156,6 +156,8 @@ __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnList
         uint32_t peer_free = 0;
         if (sid < N) peer_free = rn_mapa(bar0 + 48u, uint32_t(sid));
 
+        rn_wait_for_front();                               // the lists are there
+
         // x of the block that comes next: requested a block ahead, kept as loaded until it is put into shared memory
         RnRaw4<T> xr[XT], dr[Y ? 1 : XT];
         const T *dy = Y ? nullptr : static_cast<const T *>(p.dy) + b * p.dyb + h * p.dyh + ch;
@@ -279,6 +281,7 @@ __global__ void __launch_bounds__(RN_AP_THREADS, 1) rn_apply_kernel(const RnList
         const int lq = 31 - __clz(Lq);
         {   // the rows into shared memory, eight requests of a thread at a time; the service warps fetch the first step meanwhile
             constexpr int LD = CS / 4, STEP = RN_AP_COMPUTE / LD;
+            if (touch != nullptr) rn_wait_for_front();     // the touched rows are the gains kernel's
             const int sub = tid % LD, ch = grp * CS + sub * 4;
             const float *src = p.slot_in && ch < C ? p.slot_in + int64_t(bh) * p.A * C + ch : nullptr;
 #pragma unroll 1
@@ -521,13 +524,15 @@ static int rn_launch_apply_t(const RnListParams &p, const RnListPlan &pl, cudaSt
     cfg.blockDim = dim3(RN_AP_THREADS);
     cfg.dynamicSmemBytes = pl.smem_apply;
     cfg.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = unsigned(pl.N);
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = unsigned(pl.N);
+    at[1].val.clusterDim.y = 1;
+    at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = MODE != RN_REPLAY && pl.N > 1 ? 1 : 0;
+    cfg.numAttrs = MODE != RN_REPLAY && pl.N > 1 ? 2 : 1;
     RN_CUDA(cudaLaunchKernelEx(&cfg, rn_apply_kernel<T, CS, MODE>, p));
     return 0;
 }

@@ -320,6 +320,7 @@ __global__ void __launch_bounds__(RN_LISTS_THREADS, 1) rn_replay_lists_kernel(co
     }
 #pragma unroll 1
     for (int i = tid; i < nsteps * N; i += NT) (i < N ? first[i * p.nblocks] : table[i]).z |= uint32_t(nsteps);
+    rn_let_next_start();  // not earlier: the next kernel's blocks would crowd on the SMs that are done first
     if (tid == 0) rn_bulk_wait_read();
 }
 

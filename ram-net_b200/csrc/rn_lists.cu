@@ -362,6 +362,7 @@ __global__ void __launch_bounds__(RN_LISTS_THREADS, 1) rn_lists_kernel(const RnL
     }
 #pragma unroll 1
     for (int i = tid; i < nsteps * N; i += NT) (i < N ? first[i * p.nblocks] : table[i]).z |= uint32_t(nsteps);
+    rn_let_next_start();  // not earlier: the next kernel's blocks would crowd on the SMs that are done first
     if (tid == 0) rn_bulk_wait_read();
 }
 
@@ -399,11 +400,7 @@ __global__ void __launch_bounds__(RN_GAINS_THREADS) rn_gains_kernel(const RnList
         rn_mbar_expect_tx(&mbar[step & 1], bytes);
         rn_bulk_g2s(buf + size_t(step & 1) * p.whole_max, recs + blk * p.blk_bytes + data_at + (size_t(e.x & 0xffffu) << 4), bytes, &mbar[step & 1]);
     };
-    int blk = 0, st = 0;
-    uint4 cur = rn_step_entry(p, first, recs, 0, 0, own);
-    if (tid == 0) fetch(0, 0, cur);
-    int nblk = rn_steps_of(cur) > 1 ? 0 : 1, nst = rn_steps_of(cur) > 1 ? 1 : 0;
-    uint4 nxt = rn_step_entry(p, first, recs, nblk, nst, own);
+    if (!MA) rn_let_next_start();  // a cluster that exchanges sums every step is slowed by early neighbours
     const float *mass_in = p.mass_in ? p.mass_in + int64_t(bh) * A : nullptr;
     if (p.touch != nullptr)
         for (int i = tid; i < 2 * RN_LST_ROWS / 32; i += NT) touched[0][i] = 0;  // both rows of the array
@@ -415,6 +412,13 @@ __global__ void __launch_bounds__(RN_GAINS_THREADS) rn_gains_kernel(const RnList
         const int a = rn_slot_of<LG>(own, r);
         mass[r] = mass_in == nullptr ? p.mass_init : a < A ? mass_in[a] : 0.f;
     }
+
+    rn_wait_for_front();
+    int blk = 0, st = 0;
+    uint4 cur = rn_step_entry(p, first, recs, 0, 0, own);
+    if (tid == 0) fetch(0, 0, cur);
+    int nblk = rn_steps_of(cur) > 1 ? 0 : 1, nst = rn_steps_of(cur) > 1 ? 1 : 0;
+    uint4 nxt = rn_step_entry(p, first, recs, nblk, nst, own);
 
     bool failed = false;
     for (int step = 0; blk < p.nblocks; ++step) {
@@ -626,13 +630,15 @@ static int rn_launch_gains(const RnListParams &p, const RnListPlan &pl, cudaStre
     cfg.blockDim = dim3(RN_GAINS_THREADS);
     cfg.dynamicSmemBytes = pl.smem_gains;
     cfg.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 1u << LG;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = 1u << LG;
+    at[1].val.clusterDim.y = 1;
+    at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = MA && LG > 0 ? 1 : 0;
+    cfg.numAttrs = MA && LG > 0 ? 2 : 1;
     RN_CUDA(cudaLaunchKernelEx(&cfg, rn_gains_kernel<LG, MA>, p));
     return 0;
 }

@@ -159,6 +159,11 @@ __device__ __forceinline__ uint4 rn_step_entry(const RnListParams &p, const uint
 
 __device__ __forceinline__ int rn_steps_of(const uint4 &e) { return int(e.z & 0xffffu); }
 
+// The gains and the apply kernel are launched while the kernel in front still runs (programmatic dependent launch): they set up
+// their barriers, masses and rows, which that kernel does not write, and wait before they touch its lists.
+__device__ __forceinline__ void rn_wait_for_front() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void rn_let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- cluster primitives -----------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t rn_mapa(uint32_t addr, uint32_t rank) {
     uint32_t r;
