@@ -634,11 +634,12 @@ __global__ void __launch_bounds__(RN_SCHED_THREADS_MAX) rn_gsu_scalar_bwd_kernel
 // ------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------
-// The event lists cost two launches and a pass over the events before the sweep itself, which takes two thirds of the time of
-// the one in this file (U2 P64 K16 C128 bf16, 128 heads of 16384 tokens: 12.7 ms against 8.2 + 1.2).  So they pay where the
-// sweep is throughput bound: enough CTAs for every SM.
-static bool rn_replay_by_lists(const RnListPlan &lp, int64_t B, int64_t H, int device) {
-    return B * H * lp.ngroups * lp.N >= rn_sm_count(device);
+// The event lists cost a launch and a pass over the events before the sweep itself, which takes two thirds of the time of
+// the one in this file (U2 P64 K16 C128 bf16, 128 heads of 16384 tokens: 12.7 ms against 7.9 + 1.1).  So they pay where the
+// sweep is throughput bound, that is with a CTA for most SMs, and where it is long enough to make up for the launch: 64 heads of
+// 64 tokens lose 4 % of a training pass at K = 16, 32 heads of 500 tokens gain 7 %.
+static bool rn_replay_by_lists(const RnListPlan &lp, int64_t B, int64_t H, int64_t T, int64_t K, int device) {
+    return 3 * B * H * lp.ngroups * lp.N >= 2 * rn_sm_count(device) && T * K >= 3072;
 }
 
 struct RnBwdLayout {
@@ -649,7 +650,7 @@ struct RnBwdLayout {
 
 static void rn_bwd_layout(const RnGsuPlan &pl, int64_t B, int64_t H, int64_t T, int64_t A, int64_t C, int64_t Kw, int64_t Kr, int device,
                           RnBwdLayout *lo) {
-    lo->lists = rn_replay_plan(B, H, T, A, C, Kw, Kr, &lo->replay) && rn_replay_by_lists(lo->replay, B, H, device);
+    lo->lists = rn_replay_plan(B, H, T, A, C, Kw, Kr, &lo->replay) && rn_replay_by_lists(lo->replay, B, H, T, Kw + Kr, device);
     size_t off = 0;
     auto take = [&](size_t *at, size_t bytes) {
         *at = off;
